@@ -37,6 +37,7 @@ SOURCES = {
     "mfe_adjoint.cu": [],
     "mfe_stencil.cu": [],
     "mfe_stencil64.cu": [],
+    "mfe_fixed64.cu": [],
     "mfe_cg.cu": [],
 }
 

@@ -395,7 +395,7 @@ static mfe_status launch_cg_spmv(mfe_ctx* ctx, const mfe_csr* A, const CgBufs& B
   sink.partials = rb.partials;
   sink.ticket = rb.tickets;
   sink.out = rb.scalars;
-  if (B.st64) return launch_spmv_st64(ctx, A, B.w8, B.dd, B.p, B.Ap, &sink, B.st);
+  if (B.st64) return launch_cg_fixed(ctx, A, B.w8, B.dd, B.p, B.Ap, &sink, B.st);
   if (B.sell) return launch_spmv_sell(ctx, B.sell, B.p, B.Ap, &sink, B.st);
   return launch_spmv(ctx, A, B.p, B.Ap, &sink, nullptr, B.st);
 }

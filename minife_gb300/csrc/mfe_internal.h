@@ -181,6 +181,12 @@ mfe_status stencil64_verify_on(mfe_ctx* ctx, cudaStream_t s, int Nx, int Ny, int
 mfe_status launch_spmv_st64(mfe_ctx* ctx, const mfe_csr* A, const double* w8, double dd,
                             const double* x, double* y, const DotSink* sink, void* cg_state);
 
+// ---- the FP64 CG's product in fixed point (mfe_fixed64.cu) ----
+// Ap = S p with the same operator on the integer pipe, p.Ap and the breakdown
+// pre-test into the CG state
+mfe_status launch_cg_fixed(mfe_ctx* ctx, const mfe_csr* A, const double* w8, double dd, const double* p,
+                           double* Ap, const DotSink* sink, void* cg_state);
+
 // ---- mixed-precision CG (mfe_mixed.cu) ----
 // Reliable-update policy options of the mixed solvers: an update is due once
 // the recursive residual has fallen by inner_tol since the last one (0: 0.01,

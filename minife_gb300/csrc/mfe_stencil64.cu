@@ -1,4 +1,6 @@
-// FP64 verified stencil operator of the FP64 CG.
+// FP64 verified stencil operator: the product offered to callers
+// (mfe_spmv_stencil64) and the Jacobi PCG's.  (The FP64 CG applies the same
+// operator in fixed point, mfe_fixed64.cu.)
 //
 // On GB300 the FP64 pipe (1.9 FMA per clock per SM, 1/64 of the FP32 rate)
 // bounds the CSR SpMV of miniFE's matrix: one FP64 FMA per nonzero, 27 per
