@@ -38,6 +38,7 @@ SOURCES = {
     "mfe_stencil.cu": [],
     "mfe_stencil64.cu": [],
     "mfe_fixed64.cu": [],
+    "mfe_cg_loop.cu": [],
     "mfe_cg.cu": [],
 }
 

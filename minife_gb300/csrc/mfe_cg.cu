@@ -580,6 +580,17 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
       MFE_TRY(stencil64_prepare(ctx, &A, B.w8, &B.dd, &B.st64));  // overwrites hs
   }
 
+  // MFE_CG_EAGER=1 issues the kernels of an iteration as ordinary launches
+  // from the host (one small state read per iteration) instead of the
+  // device-side loops: identical work, visible to per-kernel profilers that do
+  // not descend into conditional graph nodes
+  const bool eager = getenv("MFE_CG_EAGER") != nullptr;
+  // Short iterations run in one cooperative kernel instead of the graph
+  // (mfe_cg_loop.cu).  Where the lines lie, us per iteration, graph against
+  // loop: CSR values 96^3 81.8 / 80.7 and 112^3 112.8 / 116.3; stencil
+  // operator 112^3 57.4 / 51.4, 128^3 73.1 / 72.5 and 144^3 90.9 / 94.1.
+  const bool loop = !eager && getenv("MFE_SPMV_GENERIC") == nullptr && !sell && csr_is_box(&A) &&
+                    A.dtype == MFE_F64 && n <= (B.st64 ? 2000000 : 1000000);
   // (re)build the graph when the operands changed
   const void* key[12] = {A.row_offsets, A.cols, A.vals, x, b, B.r, B.p, B.Ap, B.st,
                          (const void*)(uintptr_t)(((int64_t)A.box_nx << 42) ^
@@ -589,8 +600,9 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
   double op[10] = {B.st64 ? 1.0 : 0.0, B.dd};
   for (int c = 0; c < 8; ++c) op[2 + c] = B.w8[c];
   mfe_cg_graph* g = ctx->cg_graph;
-  if (!g || g->n != n || g->stream != ctx->stream || memcmp(g->key, key, sizeof(key)) != 0 ||
-      memcmp(g->op, op, sizeof(op)) != 0) {
+  if (!eager && !loop &&
+      (!g || g->n != n || g->stream != ctx->stream || memcmp(g->key, key, sizeof(key)) != 0 ||
+       memcmp(g->op, op, sizeof(op)) != 0)) {
     cg_graph_destroy(g);
     ctx->cg_graph = nullptr;
     MFE_TRY(build_graph(ctx, &A, x, B, rb, &g));
@@ -604,11 +616,6 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
   int status = MFE_OK;
   bool confirmed = spec == nullptr;
   double true_resid = -1.0;    // ||b - A x|| with the CSR values (stencil solves)
-  // MFE_CG_EAGER=1 issues the same three kernels per iteration as ordinary
-  // launches from the host (one small state read per iteration) instead of
-  // the graph's device-side loop: identical work, visible to per-kernel
-  // profilers that do not descend into conditional graph nodes
-  const bool eager = getenv("MFE_CG_EAGER") != nullptr;
   for (int restarts = 0;; ++restarts) {
     for (int round = 0;; ++round) {
       if (eager) {
@@ -620,6 +627,9 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
           MFE_TRY(launch_cg_spmv(ctx, &A, B, rb));
           MFE_TRY(launch_cg_update(ctx, n, x, B, rb, 0, 0));
         }
+      } else if (loop) {
+        const CgLoopArgs args{x, B.r, B.p, B.Ap, B.st, B.st64 ? B.w8 : nullptr, B.dd};
+        MFE_TRY(launch_cg_loop(ctx, &A, args));
       } else {
         MFE_CUDA_TRY(ctx, cudaGraphLaunch(g->exec, ctx->stream));
       }

@@ -187,6 +187,21 @@ mfe_status launch_spmv_st64(mfe_ctx* ctx, const mfe_csr* A, const double* w8, do
 mfe_status launch_cg_fixed(mfe_ctx* ctx, const mfe_csr* A, const double* w8, double dd, const double* p,
                            double* Ap, const DotSink* sink, void* cg_state);
 
+// ---- the FP64 CG's loop as one cooperative kernel (mfe_cg_loop.cu) ----
+// Iterations from the CG state until its loop test or the breakdown pre-test
+// ends them, on a box matrix: with the CSR values (w8 null) or the verified
+// stencil operator (its weights and Dirichlet diagonal).
+struct CgLoopArgs {
+  double* x;
+  double* r;
+  double* p;
+  double* Ap;
+  void* st;
+  const double* w8;
+  double dd;
+};
+mfe_status launch_cg_loop(mfe_ctx* ctx, const mfe_csr* A, const CgLoopArgs& a);
+
 // ---- mixed-precision CG (mfe_mixed.cu) ----
 // Reliable-update policy options of the mixed solvers: an update is due once
 // the recursive residual has fallen by inner_tol since the last one (0: 0.01,
