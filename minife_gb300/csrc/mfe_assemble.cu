@@ -90,12 +90,15 @@ __global__ void __launch_bounds__(kStructRows)
 // ---------------------------------------------------------------------------
 // element pass
 // ---------------------------------------------------------------------------
-constexpr int kElemThreads = 128;
+constexpr int kElemThreads = 128, kElemBlocks = 3;  // blocks per SM
+constexpr size_t kElemSmem = sizeof(double) * 44 * kElemThreads;  // em and ev, a column per thread
 constexpr int kSlab = 16;  // element planes per slab; the ring holds kSlab + 1
 
 // Per-axis Jacobian columns: jc[(base_axis + i) * 24 + gp * 3 + a] for
 // element index i along the axis (base: 0 for x, nx for y, nx + ny for z),
-// with the coordinate pair of elem_corner().
+// with the element's coordinate pair (get_elem_nodes_and_coords,
+// ref/src/Hex8_box_utils.hpp:101-159 with get_coords, box_utils.hpp:64-82): node
+// 0 at i / n, the others at + h = 1 / n.
 __global__ void k_jcols(int nx, int ny, int nz, double* __restrict__ jc)
 {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -128,11 +131,29 @@ __global__ void k_jcols(int nx, int ny, int nz, double* __restrict__ jc)
   o[2] = col[2];
 }
 
+// the Jacobian of element (ex, ey, ez) at a Gauss point, from k_jcols' table
+struct JacobianColumns {
+  const double *cx, *cy, *cz;
+  __device__ __forceinline__ JacobianColumns(const double* jc, int nx, int ny, int ex, int ey, int ez)
+      : cx(jc + (int64_t)ex * 24), cy(jc + ((int64_t)nx + ey) * 24), cz(jc + ((int64_t)nx + ny + ez) * 24)
+  {
+  }
+  __device__ __forceinline__ void operator()(int gp, double J[9]) const
+  {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      J[3 * a] = __ldg(cx + gp * 3 + a);
+      J[3 * a + 1] = __ldg(cy + gp * 3 + a);
+      J[3 * a + 2] = __ldg(cz + gp * 3 + a);
+    }
+  }
+};
+
 // Elements of planes ez0 .. ez0 + nplanes - 1 in BoxIterator order (x
 // fastest).  Element (ex, ey, ez) goes to ring index ri = ((ez mod R) ny + ey)
 // nx + ex: ke[k * RS + ri] (k < 36, upper triangle), fe[k * RS + ri] (k < 8),
 // RS = R nx ny.  kappa (nullable) is indexed by the global element id.
-__global__ void __launch_bounds__(kElemThreads)
+__global__ void __launch_bounds__(kElemThreads, kElemBlocks)
     k_element(int nx, int ny, int nz, int ez0, int nplanes, int R, const double* __restrict__ kappa,
               const double* __restrict__ jc, double* __restrict__ ke, double* __restrict__ fe)
 {
@@ -146,28 +167,14 @@ __global__ void __launch_bounds__(kElemThreads)
   const int64_t RS = (int64_t)R * nxny;
   const int64_t ri = ((int64_t)(ez % R) * ny + ey) * nx + ex;
   const double k = kappa ? kappa[e] : 1.0;
-  const double* cx = jc + (int64_t)ex * 24;
-  const double* cy = jc + ((int64_t)nx + ey) * 24;
-  const double* cz = jc + ((int64_t)nx + ny + ez) * 24;
-  double em[36], ev[8];
-  element_matrix_vector_j(
-      c_hex8,
-      [&](int gp, double J[9]) {
-        J[0] = __ldg(cx + gp * 3);
-        J[3] = __ldg(cx + gp * 3 + 1);
-        J[6] = __ldg(cx + gp * 3 + 2);
-        J[1] = __ldg(cy + gp * 3);
-        J[4] = __ldg(cy + gp * 3 + 1);
-        J[7] = __ldg(cy + gp * 3 + 2);
-        J[2] = __ldg(cz + gp * 3);
-        J[5] = __ldg(cz + gp * 3 + 1);
-        J[8] = __ldg(cz + gp * 3 + 2);
-      },
-      k, em, ev);
+  extern __shared__ double s_elem[];
+  double* const em = s_elem + threadIdx.x;
+  double* const ev = em + 36 * kElemThreads;
+  element_matrix_vector_j<kElemThreads>(c_hex8, JacobianColumns(jc, nx, ny, ex, ey, ez), k, em, ev);
 #pragma unroll
-  for (int i = 0; i < 36; ++i) ke[i * RS + ri] = em[i];
+  for (int i = 0; i < 36; ++i) ke[i * RS + ri] = em[i * kElemThreads];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) fe[i * RS + ri] = ev[i];
+  for (int i = 0; i < 8; ++i) fe[i * RS + ri] = ev[i * kElemThreads];
 }
 
 // ---------------------------------------------------------------------------
@@ -446,9 +453,9 @@ __global__ void k_ver_node(VerifyAxes A, const double* __restrict__ U, const dou
 // ---------------------------------------------------------------------------
 // adjoint contraction: g[e] = -lambda_e^T Khat_e u_e (k = 1 element matrix)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kElemThreads)
-    k_elem_grad(int nx, int ny, int nz, int64_t E, const double* __restrict__ u,
-                const double* __restrict__ lam, double* __restrict__ g)
+__global__ void __launch_bounds__(kElemThreads, kElemBlocks)
+    k_elem_grad(int nx, int ny, int nz, int64_t E, const double* __restrict__ jc,
+                const double* __restrict__ u, const double* __restrict__ lam, double* __restrict__ g)
 {
   const int64_t e = (int64_t)blockIdx.x * kElemThreads + threadIdx.x;
   if (e >= E) return;
@@ -460,9 +467,10 @@ __global__ void __launch_bounds__(kElemThreads)
   const int64_t n0 = ex + (int64_t)Nx * ey + NxNy * ez;
   const int64_t ids[8] = {n0, n0 + 1, n0 + Nx + 1, n0 + Nx,
                           n0 + NxNy, n0 + 1 + NxNy, n0 + Nx + NxNy + 1, n0 + Nx + NxNy};
-  const ElemCorner c = elem_corner(ex, ey, ez, nx, ny, nz);
-  double em[36], ev[8];
-  element_matrix_vector(c_hex8, c, 1.0, em, ev);
+  extern __shared__ double s_elem[];
+  double* const em = s_elem + threadIdx.x;
+  element_matrix_vector_j<kElemThreads>(c_hex8, JacobianColumns(jc, nx, ny, ex, ey, ez), 1.0, em,
+                                        em + 36 * kElemThreads);
   double ue[8], le[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -474,7 +482,7 @@ __global__ void __launch_bounds__(kElemThreads)
   for (int m = 0; m < 8; ++m) {
     double t = 0.0;
 #pragma unroll
-    for (int n = 0; n < 8; ++n) t += em[sym_index(m, n)] * ue[n];
+    for (int n = 0; n < 8; ++n) t += em[sym_index(m, n) * kElemThreads] * ue[n];
     s += le[m] * t;
   }
   g[e] = -s;
@@ -527,6 +535,19 @@ static void fill_tables(Hex8Tables& T)
         p[5] = 0.125 * up1 * v * wp1;
         p[6] = 0.125 * up1 * vp1 * wp1;
         p[7] = 0.125 * u * vp1 * wp1;
+        const auto split = [](double m) {
+          uint64_t bits;
+          memcpy(&bits, &m, sizeof(bits));
+          return intmul_split((uint32_t)(bits >> 32), (uint32_t)bits);
+        };
+        for (int i = 0; i < 8; ++i) T.ipsi[gp][i] = split(p[i]);
+        for (int d = 0; d < 3; ++d)
+          for (int i = 0; i < 8; ++i) {
+            const int a = hex8_side(i, d == 0 ? 1 : 0), b = hex8_side(i, d == 2 ? 1 : 2);
+            const double m = std::fabs(T.grad[gp][i][d]);
+            T.mag[gp][d][a + 2 * b] = m;
+            T.imag[gp][d][a + 2 * b] = split(m);
+          }
       }
 }
 
@@ -549,6 +570,15 @@ mfe_status launch_structure(mfe_ctx* ctx, int nx, int ny, int nz, int32_t* ro, i
   return check_launch(ctx, "k_structure");
 }
 
+// the per-axis Jacobian columns of a box, in workspace
+static mfe_status jacobian_columns(mfe_ctx* ctx, int nx, int ny, int nz, double** jc)
+{
+  *jc = static_cast<double*>(workspace(ctx, "assembly.jcols", sizeof(double) * 24 * (size_t)(nx + ny + nz)));
+  if (!*jc) return fail(ctx, MFE_OOM, "assembly scratch allocation failed");
+  k_jcols<<<(unsigned)ceil_div((int64_t)(nx + ny + nz) * 8, 128), 128, 0, ctx->stream>>>(nx, ny, nz, *jc);
+  return check_launch(ctx, "k_jcols");
+}
+
 mfe_status launch_assemble(mfe_ctx* ctx, int nx, int ny, int nz, const double* kappa,
                            const int32_t* ro, double* vals, double* b, int impose_bc)
 {
@@ -556,16 +586,14 @@ mfe_status launch_assemble(mfe_ctx* ctx, int nx, int ny, int nz, const double* k
   const int64_t nxny = (int64_t)nx * ny;
   const int64_t NxNy = (int64_t)(nx + 1) * (ny + 1);
   const int R = std::min(kSlab, nz) + 1;
-  double* jc = static_cast<double*>(workspace(ctx, "assembly.jcols",
-                                              sizeof(double) * 24 * (size_t)(nx + ny + nz)));
+  double* jc = nullptr;
+  MFE_TRY(jacobian_columns(ctx, nx, ny, nz, &jc));
   double* ke = static_cast<double*>(workspace(ctx, "assembly.ring", sizeof(double) * 44 * R * nxny));
-  if (!jc || !ke) return fail(ctx, MFE_OOM, "assembly scratch allocation failed");
+  if (!ke) return fail(ctx, MFE_OOM, "assembly scratch allocation failed");
   double* fe = ke + 36 * R * nxny;
-  k_jcols<<<(unsigned)ceil_div((int64_t)(nx + ny + nz) * 8, 128), 128, 0, ctx->stream>>>(nx, ny, nz, jc);
-  MFE_TRY(check_launch(ctx, "k_jcols"));
   for (int ez0 = 0; ez0 < nz; ez0 += kSlab) {
     const int np = std::min(kSlab, nz - ez0);
-    k_element<<<(unsigned)ceil_div(nxny * np, kElemThreads), kElemThreads, 0, ctx->stream>>>(
+    k_element<<<(unsigned)ceil_div(nxny * np, kElemThreads), kElemThreads, kElemSmem, ctx->stream>>>(
         nx, ny, nz, ez0, np, R, kappa, jc, ke, fe);
     MFE_TRY(check_launch(ctx, "k_element"));
     // node planes whose elements are all in the ring: ez0 .. ez0 + np - 1,
@@ -678,8 +706,10 @@ mfe_status launch_element_gradient(mfe_ctx* ctx, int nx, int ny, int nz, const d
 {
   MFE_TRY(ensure_tables(ctx));
   const int64_t E = (int64_t)nx * ny * nz;
-  k_elem_grad<<<(unsigned)ceil_div(E, kElemThreads), kElemThreads, 0, ctx->stream>>>(
-      nx, ny, nz, E, u, lambda, g);
+  double* jc = nullptr;
+  MFE_TRY(jacobian_columns(ctx, nx, ny, nz, &jc));
+  k_elem_grad<<<(unsigned)ceil_div(E, kElemThreads), kElemThreads, kElemSmem, ctx->stream>>>(
+      nx, ny, nz, E, jc, u, lambda, g);
   return check_launch(ctx, "k_elem_grad");
 }
 

@@ -8,6 +8,8 @@
 
 #include <cstdint>
 
+#include "mfe_intmul.cuh"
+
 namespace mfe {
 
 // 2x2x2 Gauss points from gauss_pts(2) (ref/fem/gauss_pts.hpp:41,50-53): the
@@ -22,77 +24,46 @@ constexpr double kGaussPt = 0.577350269;
 struct Hex8Tables {
   double grad[8][8][3];
   double psi[8][8];  // shape_fns at each Gauss point (Hex8.hpp:44-65)
+  // |grad[gp][i][d]| depends on the node's two other sides only:
+  // mag[gp][d][a + 2 b] for sides a, b along the other two dimensions in order;
+  // and the same taken apart for integer multiplication
+  double mag[8][3][4];
+  IntMul imag[8][3][4];
+  IntMul ipsi[8][8];  // psi taken apart
 };
 
-// Element node coordinates (get_elem_nodes_and_coords,
-// ref/src/Hex8_box_utils.hpp:101-159 with get_coords, box_utils.hpp:64-82):
-// node 0 at (ex/nx, ey/ny, ez/nz), the others at + h = 1/n per dimension.
-struct ElemCorner {
-  double x0, x1, y0, y1, z0, z1;
-};
-
-__device__ __forceinline__ ElemCorner elem_corner(int ex, int ey, int ez, int nx, int ny, int nz)
+// node i's side (0 or 1) along dimension d
+__host__ __device__ constexpr int hex8_side(int i, int d)
 {
-  ElemCorner c;
-  // xdiv = Nx - 1 = nx (nx >= 1 for every assembled box)
-  c.x0 = (1.0 * (double)ex) / (double)nx;
-  c.y0 = 1.0 * (double)ey / (double)ny;
-  c.z0 = (1.0 * (double)ez) / (double)nz;
-  c.x1 = c.x0 + 1.0 / nx;
-  c.y1 = c.y0 + 1.0 / ny;
-  c.z1 = c.z0 + 1.0 / nz;
-  return c;
-}
-
-// Coordinates of local node i (get_hex8_node_coords_3d order).
-__device__ __forceinline__ void node_xyz(const ElemCorner& c, int i, double& x, double& y,
-                                         double& z)
-{
-  const bool hx = (i == 1 || i == 2 || i == 5 || i == 6);
-  const bool hy = (i == 2 || i == 3 || i == 6 || i == 7);
-  const bool hz = (i >= 4);
-  x = hx ? c.x1 : c.x0;
-  y = hy ? c.y1 : c.y0;
-  z = hz ? c.z1 : c.z0;
-}
-
-// Jacobian at one Gauss point (Hex8.hpp:198-236): J += grad * coord in node
-// order 0..7.
-__device__ __forceinline__ void jacobian(const ElemCorner& c, const double (*g)[3],
-                                         double J[9])
-{
-  double J00 = 0, J01 = 0, J02 = 0, J10 = 0, J11 = 0, J12 = 0, J20 = 0, J21 = 0, J22 = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    double x, y, z;
-    node_xyz(c, i, x, y, z);
-    const double g0 = g[i][0], g1 = g[i][1], g2 = g[i][2];
-    J00 += g0 * x; J01 += g0 * y; J02 += g0 * z;
-    J10 += g1 * x; J11 += g1 * y; J12 += g1 * z;
-    J20 += g2 * x; J21 += g2 * y; J22 += g2 * z;
-  }
-  J[0] = J00; J[1] = J01; J[2] = J02; J[3] = J10; J[4] = J11; J[5] = J12;
-  J[6] = J20; J[7] = J21; J[8] = J22;
+  return d == 0 ? (i == 1 || i == 2 || i == 5 || i == 6) : d == 1 ? (i == 2 || i == 3 || i == 6 || i == 7) : i >= 4;
 }
 
 // diffusionMatrix_symm (Hex8.hpp:260-361) with conductivity k, and
 // sourceVector (Hex8.hpp:364-410).  em: 36 upper-triangle entries, row-major;
 // ev: 8 entries.  Both loops walk the Gauss points in the same order and
 // compute the same Jacobian, so they share it.  jf(gp, J) provides the
-// Jacobian at Gauss point gp (jacobian() from the corner coordinates, or the
-// same values from per-axis tables, jacobian_column()).
-template <typename JF>
-__device__ __forceinline__ void element_matrix_vector_j(const Hex8Tables& T, JF jf, double k,
-                                                        double em[36], double ev[8])
+// Jacobian at Gauss point gp (from per-axis tables, jacobian_column()).
+// The sums lie in shared memory, entry i at em[i * S] and ev[i * S] (a column
+// per thread): 88 registers less, so that three blocks of 128 threads share an
+// SM and one warp's integer work runs beside another's FP64 work.
+// Per Gauss point that leaves 214 operations for the FP64 pipe (438 with the
+// multiplications) and about 4,000 integer instructions.  Measured, k_element
+// over 256^3 elements (16 launches): 111 ms with all of it in FP64; 72 ms with
+// the 108 products and 36 scalings of the matrix entries as integers (and 36
+// gradient products for 72); 66 ms with the gradient and source products too;
+// 61 ms with the sums in shared memory, 0.79 of the FP64 pipe's rate on what is
+// left there (four blocks of 128 registers: 62 ms).
+template <int S, typename JF>
+__device__ __forceinline__ void element_matrix_vector_j(const Hex8Tables& T, JF jf, double k, double* em,
+                                                        double* ev)
 {
 #pragma unroll
-  for (int i = 0; i < 36; ++i) em[i] = 0.0;
+  for (int i = 0; i < 36; ++i) em[i * S] = 0.0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) ev[i] = 0.0;
+  for (int i = 0; i < 8; ++i) ev[i * S] = 0.0;
 
 #pragma unroll 1
   for (int gp = 0; gp < 8; ++gp) {
-    const double (*g)[3] = T.grad[gp];
     double J[9];
     jf(gp, J);
     const double J00 = J[0], J01 = J[1], J02 = J[2], J10 = J[3], J11 = J[4], J12 = J[5],
@@ -115,42 +86,107 @@ __device__ __forceinline__ void element_matrix_vector_j(const Hex8Tables& T, JF 
 
     // weights are 1.0: wi_wj_wk = 1*1*1 (Hex8.hpp:293-299)
     const double k_detJ_w = k * detJ * 1.0;
-    double dx[8], dy[8], dz[8];
+    // The multiplications run on the integer pipe (mfe_intmul.cuh), the
+    // additions on the FP64 pipe.  detJ and k_detJ_w lie in [2^-200, 2^200] and
+    // the entries of iJ are zero or in [2^-300, 2^300] on any box worth the name,
+    // and then so are the gradients within [2^-340, 2^340]; the sums of their
+    // products are zero or at least 2^-735, and every product is a normal
+    // number.  Anything else takes the FP64 form (wide).
+    bool wide = !intmul_range<200>(k_detJ_w) || !intmul_range<200>(detJ);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const double g0 = g[i][0], g1 = g[i][1], g2 = g[i][2];
-      dx[i] = g0 * iJ[0] + g1 * iJ[1] + g2 * iJ[2];
-      dy[i] = g0 * iJ[3] + g1 * iJ[4] + g2 * iJ[5];
-      dz[i] = g0 * iJ[6] + g1 * iJ[7] + g2 * iJ[8];
-    }
-    int off = 0;
+    for (int j = 0; j < 9; ++j) wide = wide || !(iJ[j] == 0.0 || intmul_range<300>(iJ[j]));
+    // The gradients (Hex8.hpp:301-310): node i's is a sum of three products
+    // +-|g| * iJ, and |g| takes four values per dimension, so 36 products do
+    // for the 72 (a product's sign does not change its rounding).
+    double dxyz[3][8];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      em[off] += k_detJ_w * ((dx[m] * dx[m]) + (dy[m] * dy[m]) + (dz[m] * dz[m]));
-      ++off;
+    for (int c = 0; c < 3; ++c) {
+      double q[3][4];
 #pragma unroll
-      for (int n = m + 1; n < 8; ++n) {
-        em[off] += k_detJ_w * ((dx[m] * dx[n]) + (dy[m] * dy[n]) + (dz[m] * dz[n]));
-        ++off;
+      for (int d = 0; d < 3; ++d) {
+        const double f = iJ[3 * c + d];
+        const uint32_t fh = (uint32_t)__double2hiint(f), fl = (uint32_t)__double2loint(f);
+        const IntMul F = intmul_split(fh, fl);
+        const bool zero = (fh << 1) == 0u;  // (the product then is f)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          uint32_t h, l;
+          intmul(T.imag[gp][d][t], F, h, l);
+          q[d][t] = __hiloint2double((int)(zero ? fh : h), (int)(zero ? fl : l));
+        }
       }
+      if (wide) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) q[d][t] = T.mag[gp][d][t] * iJ[3 * c + d];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int sx = hex8_side(i, 0), sy = hex8_side(i, 1), sz = hex8_side(i, 2);
+        const double p0 = sx ? q[0][sy + 2 * sz] : -q[0][sy + 2 * sz];
+        const double p1 = sy ? q[1][sx + 2 * sz] : -q[1][sx + 2 * sz];
+        const double p2 = sz ? q[2][sx + 2 * sy] : -q[2][sx + 2 * sy];
+        dxyz[c][i] = p0 + p1 + p2;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) wide = wide || !intmul_range<340>(dxyz[c][i]);
+    // em += k_detJ_w * ((dx dx) + (dy dy) + (dz dz)) per pair of nodes
+    // (Hex8.hpp:312-340)
+    if (!wide) {
+      IntMul D[3][8];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) D[c][i] = intmul_split(dxyz[c][i]);
+      const IntMul K = intmul_split(k_detJ_w);
+      const uint32_t ksign = (uint32_t)__double2hiint(k_detJ_w) & 0x80000000u;
+      int off = 0;
+#pragma unroll
+      for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int n = m; n < 8; ++n) {
+          const double s = intmul(D[0][m], D[0][n]) + intmul(D[1][m], D[1][n]) + intmul(D[2][m], D[2][n]);
+          const uint32_t sh = (uint32_t)__double2hiint(s), sl = (uint32_t)__double2loint(s);
+          uint32_t ph, pl;
+          intmul(intmul_split(sh, sl), K, ph, pl);
+          if ((sh << 1) == 0u) {  // a sum of zero (none is subnormal)
+            ph = sh ^ ksign;
+            pl = 0u;
+          }
+          em[off * S] += __hiloint2double((int)ph, (int)pl);
+          ++off;
+        }
+    } else {
+      int off = 0;
+#pragma unroll
+      for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int n = m; n < 8; ++n) {
+          em[off * S] += k_detJ_w * ((dxyz[0][m] * dxyz[0][n]) + (dxyz[1][m] * dxyz[1][n]) + (dxyz[2][m] * dxyz[2][n]));
+          ++off;
+        }
     }
     // sourceVector: term = Q*detJ*wi*wj*wk with Q = 1 (Hex8.hpp:402)
     const double term = 1.0 * detJ * 1.0 * 1.0 * 1.0;
+    if (!wide) {
+      const IntMul D = intmul_split(term);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) ev[i] += T.psi[gp][i] * term;
+      for (int i = 0; i < 8; ++i) ev[i * S] += intmul(T.ipsi[gp][i], D);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ev[i * S] += T.psi[gp][i] * term;
+    }
   }
-}
-
-__device__ __forceinline__ void element_matrix_vector(const Hex8Tables& T, const ElemCorner& c,
-                                                      double k, double em[36], double ev[8])
-{
-  element_matrix_vector_j(T, [&](int gp, double J[9]) { jacobian(c, T.grad[gp], J); }, k, em, ev);
 }
 
 // The Jacobian's column for physical axis x (entries J[a][0], a = 0..2) sums
 // grad[gp][i][a] * x_i over the element's 8 nodes, whose x is x0 or x1: it
 // depends on the element's x pair only, and likewise for y and z.  Computed
-// with jacobian()'s operations in its order (node order, from 0), the column
+// with the reference's operations in its order (Hex8.hpp:198-236) (node order, from 0), the column
 // of an element index along an axis is therefore exact for every element of
 // that index.  axis: 0 x, 1 y, 2 z; (c0, c1) the index's coordinate pair.
 __device__ __forceinline__ void jacobian_column(const Hex8Tables& T, int axis, double c0, double c1,
