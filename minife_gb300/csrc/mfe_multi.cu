@@ -39,6 +39,11 @@ constexpr int kProdM = 2;       // producer warps per CTA (tiles alternate betwe
 constexpr int kThreadsM = (kConsM + kProdM) * 32;
 constexpr int kVT = 256;
 constexpr int kMaxPartM = 2048;
+// reductions (multi_dot_reduce): blocks per group, and what one needs of
+// partials (32 each) and tickets
+constexpr int kGroupM = 32;
+constexpr int kPartsM = kMaxPartM + kMaxPartM / kGroupM;
+constexpr int kTicketsM = 1 + kMaxPartM / kGroupM;
 
 // stage capacities (elements): a tile's values, and one x segment of
 // kTileRowsM + 2 rows of nrhs values, each with room for rounding both ends
@@ -102,43 +107,52 @@ struct SpmmParams {
   MultiState* cg;                // DOT mode in a solve: also set cg->alpha from out
 };
 
-// Per-lane dots of the block summed over its warps, then over blocks in
-// block order by the last block: out[j] = total of lane j.  red: >= 33*32.
-// With cg set (out = cg->pAp) the last block also forms cg->alpha.
+// Per-lane dots of the block summed over its warps, then over groups of
+// kGroupM blocks in block order by each group's last block, then over the
+// groups in order by the last group's: out[j] = total of lane j.  red: >= 32
+// per warp.  With cg set (out = cg->pAp) the last block also forms cg->alpha.
+// One block summing the partials of all (up to 1,216 x 32 of them) queued
+// 10 us on its SM's FP64 pipe: 64^3 x 32, the r update 33.5 us (cold caches),
+// with the groups 24.1.
 __device__ void multi_dot_reduce(double v, double* red, double* partials, unsigned* ticket,
                                  double* out, int nlanes, MultiState* cg = nullptr)
 {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  red[warp * 32 + lane] = v;
-  __syncthreads();
   __shared__ bool am_last;
-  if (threadIdx.x < 32) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += red[w * 32 + threadIdx.x];
-    partials[(size_t)blockIdx.x * 32 + threadIdx.x] = s;
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) am_last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  // every warp of the last block sums the partials of blocks warp,
-  // warp + nw, ... (four accumulators keep four L2 loads in flight), then
-  // the warps' sums are added in warp order: a fixed order for a fixed grid
-  {
-    const unsigned g = gridDim.x, uw = (unsigned)warp, unw = (unsigned)nw;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    unsigned bl = uw;
-    for (; bl + 3 * unw < g; bl += 4 * unw) {
-      s0 += __ldcg(&partials[(size_t)bl * 32 + lane]);
-      s1 += __ldcg(&partials[(size_t)(bl + unw) * 32 + lane]);
-      s2 += __ldcg(&partials[(size_t)(bl + 2 * unw) * 32 + lane]);
-      s3 += __ldcg(&partials[(size_t)(bl + 3 * unw) * 32 + lane]);
+  // the block's warps' sums in red, to `to`; true in the last of `count`
+  // blocks to get here
+  auto publish = [&](double* to, unsigned* t, unsigned count) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      double s = 0.0;
+      for (int w = 0; w < nw; ++w) s += red[w * 32 + threadIdx.x];
+      to[threadIdx.x] = s;
     }
-    for (; bl < g; bl += unw) s0 += __ldcg(&partials[(size_t)bl * 32 + lane]);
-    red[warp * 32 + lane] = (s0 + s1) + (s2 + s3);
-  }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      am_last = atomicAdd(t, 1u) == count - 1;
+      if (am_last) *t = 0u;
+    }
+    __syncthreads();
+    if (am_last) __threadfence();
+    return am_last;
+  };
+  // `count` sums of 32 from `from` on, into red: the warps take every nw-th
+  auto gather = [&](const double* from, int count) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = warp; i < count; i += nw) s += __ldcg(&from[(size_t)i * 32 + lane]);
+    red[warp * 32 + lane] = s;
+  };
+  const int g = (int)blockIdx.x / kGroupM, ng = ((int)gridDim.x + kGroupM - 1) / kGroupM;
+  const int members = min(kGroupM, (int)gridDim.x - g * kGroupM);
+  double* const groups = partials + (size_t)kMaxPartM * 32;
+  red[warp * 32 + lane] = v;
+  if (!publish(partials + (size_t)blockIdx.x * 32, ticket + 1 + g, (unsigned)members)) return;
+  gather(partials + (size_t)g * kGroupM * 32, members);
+  if (!publish(groups + (size_t)g * 32, ticket, (unsigned)ng)) return;
+  gather(groups, ng);
   __syncthreads();
   if (threadIdx.x < nlanes) {
     double s = 0.0;
@@ -147,7 +161,6 @@ __device__ void multi_dot_reduce(double v, double* red, double* partials, unsign
     if (cg)
       cg->alpha[threadIdx.x] = cg->done[threadIdx.x] || !(s > 0.0) ? 0.0 : cg->rr[threadIdx.x] / s;
   }
-  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // NRC: nrhs as a compile-time constant (32), or 0 to read it from P
@@ -669,7 +682,27 @@ __global__ void __launch_bounds__(kEThreads, 2) k_spmm_ell32(Ell32Params P)
 // ---------------------------------------------------------------------------
 constexpr int kSMW = 8;    // warps per CTA
 constexpr int kSMKP = 4;   // positions per warp
-constexpr int kSMZC = 32;  // default z steps per work item (mfe_multi_set_tuning)
+
+// z steps per work item where the caller sets none (mfe_multi_set_tuning): an
+// item marches its steps and two planes more, and every resident warp takes an
+// equal number of items, so the chunks that make the busiest warp's planes
+// fewest.  64^3 x 32: 17 steps (one wave of 4,228 items), the product 30.5 us,
+// 41.0 with chunks of 32 (the last of one step).
+int st32_default_chunk(int64_t ntile, int Nz, int64_t warps)
+{
+  int best = Nz;
+  int64_t least = -1;
+  for (int nzc = 1; nzc <= Nz; ++nzc) {
+    const int zc = (int)ceil_div((int64_t)Nz, (int64_t)nzc);
+    const int64_t items = ntile * ceil_div((int64_t)Nz, (int64_t)zc);
+    const int64_t planes = ceil_div(items, warps) * (zc + 2);
+    if (least < 0 || planes < least) {
+      least = planes;
+      best = zc;
+    }
+  }
+  return best;
+}
 
 struct MSt32Params {
   int Nx, Ny, Nz, NxNy, ntile, nzc, zc;  // zc: z steps per work item
@@ -1259,7 +1292,7 @@ struct MultiBufs {
   V *r, *p, *Ap;
   float* x32;  // mixed only
   MultiState* st;
-  double* partials;  // [2][kMaxPartM][32]
+  double* partials;  // [2][kPartsM][32]
   unsigned* tickets;
   unsigned* err;
   const float* ell = nullptr;  // mixed, 32 right-hand sides: padded values (p has ghost zones)
@@ -1270,7 +1303,7 @@ struct MultiBufs {
   float w8[8] = {};
   float dd = 0.0f;
   int st32_grid = 0;
-  int st32_zc = kSMZC;
+  int st32_zc = 1;
 };
 
 size_t ell32_smem() { return (size_t)2 * kEStage * sizeof(float); }
@@ -1357,7 +1390,7 @@ mfe_status multi_iter_mixed(mfe_ctx* ctx, const mfe_csr& A32, const mfe_csr& A64
                                                   W.st)));
   }
   k_mr_update<float><<<vgrid(ctx, ntot, k_mr_update<float>), kVT, 0, ctx->stream>>>(
-      ntot, nrhs, W.x32, W.r, W.p, W.Ap, W.st, W.partials + (size_t)kMaxPartM * 32, W.tickets + 1);
+      ntot, nrhs, W.x32, W.r, W.p, W.Ap, W.st, W.partials + (size_t)kPartsM * 32, W.tickets + kTicketsM);
   MFE_TRY(check_launch(ctx, "k_mr_update"));
   k_mr_decide<<<1, 32, 0, ctx->stream>>>(W.st, h, h_upd, in_graph);
   return check_launch(ctx, "k_mr_decide");
@@ -1390,7 +1423,7 @@ mfe_status multi_iter_f64(mfe_ctx* ctx, const mfe_csr& A64, int nrhs, double* X,
                                                   W.partials, W.tickets, W.st->pAp, nullptr, W.err,
                                                   W.st)));
   k_mr_update<double><<<vgrid(ctx, ntot, k_mr_update<double>), kVT, 0, ctx->stream>>>(
-      ntot, nrhs, X, W.r, W.p, W.Ap, W.st, W.partials + (size_t)kMaxPartM * 32, W.tickets + 1);
+      ntot, nrhs, X, W.r, W.p, W.Ap, W.st, W.partials + (size_t)kPartsM * 32, W.tickets + kTicketsM);
   MFE_TRY(check_launch(ctx, "k_mr_update"));
   k_mr_after64<<<1, 32, 0, ctx->stream>>>(W.st, h, in_graph);
   return check_launch(ctx, "k_mr_after64");
@@ -1575,14 +1608,14 @@ mfe_status cg_multi(mfe_ctx* ctx, const mfe_csr* A64_in, int nrhs, const double*
     A32.dtype = MFE_F32;
   }
   int st32_grid = 0;
-  const int st32_zc = ctx->multi_zchunk > 0 ? ctx->multi_zchunk : kSMZC;
+  int st32_zc = ctx->multi_zchunk;
   if (use_st32) {
-    const int64_t items = ceil_div((int64_t)(A64.box_nx + 1) * (A64.box_ny + 1), (int64_t)kSMKP) *
-                          ceil_div((int64_t)(A64.box_nz + 1), (int64_t)st32_zc);
-    st32_grid = (int)std::max<int64_t>(
-        1, std::min<int64_t>({ceil_div(items, (int64_t)kSMW),
-                              (int64_t)resident_blocks(ctx, (const void*)k_spmm_st32, kSMW * 32, 0),
-                              (int64_t)kMaxPartM}));
+    const int64_t blocks = std::min<int64_t>(
+        resident_blocks(ctx, (const void*)k_spmm_st32, kSMW * 32, 0), (int64_t)kMaxPartM);
+    const int64_t ntile = ceil_div((int64_t)(A64.box_nx + 1) * (A64.box_ny + 1), (int64_t)kSMKP);
+    if (st32_zc <= 0) st32_zc = st32_default_chunk(ntile, A64.box_nz + 1, blocks * kSMW);
+    const int64_t items = ntile * ceil_div((int64_t)(A64.box_nz + 1), (int64_t)st32_zc);
+    st32_grid = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(items, (int64_t)kSMW), blocks));
   }
   const size_t vb = (mixed ? sizeof(float) : sizeof(double)) * (size_t)(ntot + 8);
   void* r = workspace(ctx, "multi.r", vb);
@@ -1610,13 +1643,13 @@ mfe_status cg_multi(mfe_ctx* ctx, const mfe_csr* A64_in, int nrhs, const double*
   float* x32 = mixed ? static_cast<float*>(workspace(ctx, "multi.x32", vb)) : nullptr;
   MultiState* dst = static_cast<MultiState*>(workspace(ctx, "multi.state", sizeof(MultiState)));
   double* partials =
-      static_cast<double*>(workspace(ctx, "multi.partials", sizeof(double) * 2 * kMaxPartM * 32));
+      static_cast<double*>(workspace(ctx, "multi.partials", sizeof(double) * 2 * kPartsM * 32));
   const bool fresh = ctx->ws.find("multi.tickets") == ctx->ws.end();
-  unsigned* tickets = static_cast<unsigned*>(workspace(ctx, "multi.tickets", sizeof(unsigned) * 4));
+  unsigned* tickets = static_cast<unsigned*>(workspace(ctx, "multi.tickets", sizeof(unsigned) * 2 * kTicketsM));
   unsigned* err = static_cast<unsigned*>(workspace(ctx, "multi.err", sizeof(unsigned)));
   if (!r || !pbase || !Ap || (mixed && !x32) || !dst || !partials || !tickets || !err)
     return fail(ctx, MFE_OOM, "multi-RHS workspace allocation failed");
-  if (fresh) MFE_CUDA_TRY(ctx, cudaMemsetAsync(tickets, 0, sizeof(unsigned) * 4, ctx->stream));
+  if (fresh) MFE_CUDA_TRY(ctx, cudaMemsetAsync(tickets, 0, sizeof(unsigned) * 2 * kTicketsM, ctx->stream));
   MFE_CUDA_TRY(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
 
   MultiState* hs = static_cast<MultiState*>(host_scratch(ctx, sizeof(MultiState) + 64));
