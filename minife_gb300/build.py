@@ -39,6 +39,7 @@ SOURCES = {
     "mfe_stencil64.cu": [],
     "mfe_fixed64.cu": [],
     "mfe_cg_loop.cu": [],
+    "mfe_graph.cu": [],
     "mfe_cg.cu": [],
 }
 

@@ -1205,6 +1205,7 @@ __global__ void __launch_bounds__(1024)
     k_bx_after(const BoxDesc* boxes, BoxSt* st, BatchCtl* ctl, BxList open,
                cudaGraphConditionalHandle h, int in_graph)
 {
+  if (ctl->cont == 0) return;  // the loop ended in an earlier iteration of its body
   const int b = threadIdx.x;
   const int nbox = ctl->nbox;
   const int k = ctl->k + 1;
@@ -1266,6 +1267,7 @@ __global__ void __launch_bounds__(1024)
     k_bx_after64(const BoxDesc* boxes, BoxSt* st, BatchCtl* ctl, BxList open,
                  cudaGraphConditionalHandle h, int in_graph)
 {
+  if (ctl->cont == 0) return;  // the loop ended in an earlier iteration of its body
   const int b = threadIdx.x;
   const int nbox = ctl->nbox;
   const int k = ctl->k + 1;
@@ -1592,51 +1594,17 @@ mfe_status bx_loop(mfe_ctx* ctx, BatchCtl* dctl, Body body)
       MFE_TRY(body((cudaGraphConditionalHandle)0, 0));
     }
   }
-  cudaStream_t run_stream = ctx->stream, s = ctx->own_stream;
-  cudaGraph_t g = nullptr;
-  cudaGraphExec_t ex = nullptr;
-  cudaGraphConditionalHandle h = 0;
-  mfe_status st = MFE_OK;
-  cudaError_t e = cudaGraphCreate(&g, 0);
-  if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-  if (e == cudaSuccess) {
-    ctx->stream = s;
-    e = cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-    if (e == cudaSuccess) {
-      k_bx_begin<<<1, 1, 0, s>>>(dctl, h);
-      e = cudaStreamEndCapture(s, &g);
-    }
-    cudaGraphNode_t nodes[4];
-    size_t nn = 4;
-    if (e == cudaSuccess) e = cudaGraphGetNodes(g, nodes, &nn);
-    alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)];
-    memset(cp_buf, 0, sizeof(cp_buf));
-    cudaGraphNodeParams* cp = reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
-    cp->type = cudaGraphNodeTypeConditional;
-    cp->conditional.handle = h;
-    cp->conditional.type = cudaGraphCondTypeWhile;
-    cp->conditional.size = 1;
-    cudaGraphNode_t cnode;
-    if (e == cudaSuccess) e = cudaGraphAddNode(&cnode, g, &nodes[0], nullptr, 1, cp);
-    if (e == cudaSuccess) {
-      cudaGraph_t bg = cp->conditional.phGraph_out[0];
-      e = cudaStreamBeginCaptureToGraph(s, bg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-      if (e == cudaSuccess) {
-        st = body(h, 1);
-        cudaGraph_t tmp;
-        const cudaError_t e2 = cudaStreamEndCapture(s, &tmp);
-        if (e == cudaSuccess) e = e2;
-      }
-    }
-    ctx->stream = run_stream;
-    if (e == cudaSuccess && st == MFE_OK) e = cudaGraphInstantiate(&ex, g, 0);
-    if (e == cudaSuccess && st == MFE_OK) e = cudaGraphLaunch(ex, ctx->stream);
-  }
-  if (ex) cudaGraphExecDestroy(ex);
-  if (g) cudaGraphDestroy(g);
-  if (st != MFE_OK) return st;
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "batched CG graph");
-  return MFE_OK;
+  GraphLoop L;
+  L.begin = [&](cudaGraphConditionalHandle h) {
+    k_bx_begin<<<1, 1, 0, ctx->stream>>>(dctl, h);
+    return check_launch(ctx, "k_bx_begin");
+  };
+  L.body = [&](cudaGraphConditionalHandle h, cudaGraphConditionalHandle) { return body(h, 1); };
+  // The kernels of a reliable update run empty where no box takes one: a
+  // conditional node per iteration for them measured 35.8 ms against 34.9
+  // (24 boxes of 16..96 to 1e-13), one iteration per test 36.0.
+  L.copies = 4;
+  return run_graph_loop(ctx, L, "batched CG graph");
 }
 
 }  // namespace

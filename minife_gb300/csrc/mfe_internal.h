@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <map>
 #include <string>
 #include <vector>
@@ -67,6 +68,22 @@ void* host_scratch(mfe_ctx* ctx, size_t bytes);
 // device.  Grid-stride kernels sized to it run in one wave instead of a full
 // wave plus a partial one.  Call it once before a graph capture.
 int resident_blocks(mfe_ctx* ctx, const void* kernel, int threads, size_t smem);
+
+// ---- device-side solver loops (mfe_graph.cu) ----
+// Runs begin, then the loop body while its condition (set by begin, the body
+// and the update on the device) holds, as one graph launch on ctx->stream.
+// The body is `copies` iterations in a row, because the while node's test
+// costs about 5 us; kernels of the iterations after the one that ended the
+// loop (or asked for the update) return at once.  update, when set, runs in a
+// conditional node after the last copy, under the condition handed to the
+// body (a conditional node costs about 5 us too).
+struct GraphLoop {
+  std::function<mfe_status(cudaGraphConditionalHandle loop)> begin;
+  std::function<mfe_status(cudaGraphConditionalHandle loop, cudaGraphConditionalHandle upd)> body;
+  std::function<mfe_status(cudaGraphConditionalHandle loop)> update;
+  int copies = 1;
+};
+mfe_status run_graph_loop(mfe_ctx* ctx, const GraphLoop& L, const char* where);
 
 // ---- assembly (mfe_assemble.cu) ----
 mfe_status launch_structure(mfe_ctx* ctx, int nx, int ny, int nz, int32_t* ro, int32_t* cols);
@@ -146,9 +163,11 @@ bool stencil_mirror_classes(const float* coef, float* w8);
 mfe_status stencil_grid(mfe_ctx* ctx, const float* coef, int* grid);
 // y = S x and x.y into sink->out (the eight class weights when the stencil
 // is mirror-symmetric, else the 27 coefficients), both x-padded (y's padding entries are
-// written as zeros); x has stencil_ghost rows of zeros on both sides
+// written as zeros); x has stencil_ghost rows of zeros on both sides; the
+// launch does nothing when run is set and *run == 0 (read on the device)
 mfe_status launch_spmv_stencil(mfe_ctx* ctx, const mfe_csr* A, const float* coef, const float* x,
-                               float* y, const DotSink* sink, int grid, unsigned* err);
+                               float* y, const DotSink* sink, int grid, unsigned* err,
+                               const int* run = nullptr);
 
 // ---- FP64 stencil operator of the FP64 CG (mfe_stencil64.cu; its check in
 // mfe_stencil.cu) ----

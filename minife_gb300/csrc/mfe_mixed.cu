@@ -53,6 +53,7 @@ struct MixState {
   int max_refine;       // stop after this many updates (0: no cap)
   int gate;             // 1: a reliable update runs in this iteration
   int cont;             // loop condition
+  int run;              // 0: the rest of the loop body's iterations do nothing
   int first;            // next p update is p = r
   int updates;          // reliable updates done
   int status;           // 0 ok, MFE_BREAKDOWN
@@ -65,6 +66,9 @@ struct MixState {
 
 constexpr int kT = 256;
 constexpr int kMaxPart = 8192;
+// iterations in a row in the loop's body (160 x 192 x 144, us per iteration: 1
+// 46.5, 2 43.5, 4 41.6, 8 40.9; 40^3: 22.7, 19.7, 18.1, 17.6)
+constexpr int kCopies = 8;
 
 // p = r (first) or p = r + beta p, FP32 (cg_solve.hpp:153-161).  The previous
 // iteration's x32 += alpha p (cg_solve.hpp:201-205) is done here, where the
@@ -74,6 +78,7 @@ __global__ void __launch_bounds__(kT)
     k_mx_p(int64_t n, const float* __restrict__ r, float* __restrict__ p, float* __restrict__ x32,
            const MixState* st)
 {
+  if (st->run == 0) return;
   const bool first = st->first != 0;
   const bool addx = !first && st->x_pending != 0;
   const float beta = (float)st->beta;
@@ -125,6 +130,7 @@ __global__ void __launch_bounds__(kT)
 {
   __shared__ float2 red[32];
   __shared__ float s_alpha;
+  if (st->run == 0) return;
   if (threadIdx.x == 0) s_alpha = st->pAp > 0.0 ? (float)(st->rr / st->pAp) : 0.0f;
   __syncthreads();
   const float alpha = s_alpha;
@@ -176,6 +182,7 @@ __global__ void __launch_bounds__(kT)
         }
         cudaGraphSetConditional(h_loop, st->cont ? 1u : 0u);
       }
+      st->run = st->cont && !st->gate;
       cudaGraphSetConditional(h_upd, st->gate ? 1u : 0u);
     }
   }
@@ -223,6 +230,7 @@ __global__ void k_mx_after(MixState* st, cudaGraphConditionalHandle h, int in_gr
     st->cont = st->k < st->max_iter;
   }
   st->gate = 0;
+  st->run = st->cont;
   if (in_graph) cudaGraphSetConditional(h, st->cont ? 1u : 0u);
 }
 
@@ -237,6 +245,7 @@ __global__ void k_mx_init(MixState* st)
   st->rr = st->rr_true;
   st->rr_at_update = st->rr_true;
   st->cont = (st->max_iter > 0) && (nr > st->tol_abs);
+  st->run = st->cont;
   if (st->record) st->history[0] = nr;
 }
 
@@ -286,7 +295,7 @@ mfe_status launch_iter(mfe_ctx* ctx, const mfe_csr& A32, const mfe_csr& A64, con
   s1.ticket = B.tickets;
   s1.out = &B.st->pAp;
   if (B.stencil)
-    MFE_TRY(launch_spmv_stencil(ctx, &A32, B.coef, B.p, B.Ap, &s1, B.stencil_grid, B.err));
+    MFE_TRY(launch_spmv_stencil(ctx, &A32, B.coef, B.p, B.Ap, &s1, B.stencil_grid, B.err, &B.st->run));
   else
     MFE_TRY(launch_spmv(ctx, &A32, B.p, B.Ap, &s1, nullptr, nullptr));
   k_mx_update<<<grid_for(ctx, nv / 4, (const void*)k_mx_update), kT, 0, ctx->stream>>>(
@@ -433,89 +442,19 @@ mfe_status cg_mixed(mfe_ctx* ctx, const mfe_csr* A64_in, const double* b, double
       MFE_TRY(launch_update(ctx, A64, b, x, B, 0, 0));
     }
   } else {
-    // graph: begin kernel, then while(cont) { one iteration }
-    cudaStream_t run_stream = ctx->stream;
-    cudaStream_t s = ctx->own_stream;
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ex = nullptr;
-    cudaGraphConditionalHandle h = 0;
-    cudaError_t e = cudaGraphCreate(&g, 0);
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-    mfe_status st = MFE_OK;
-    if (e == cudaSuccess) {
-      ctx->stream = s;
-      e = cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-      if (e == cudaSuccess) {
-        k_mx_begin<<<1, 1, 0, s>>>(B.st, h);
-        e = cudaStreamEndCapture(s, &g);
-      }
-      cudaGraphNode_t nodes[4];
-      size_t nn = 4;
-      if (e == cudaSuccess) e = cudaGraphGetNodes(g, nodes, &nn);
-      alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)];
-      memset(cp_buf, 0, sizeof(cp_buf));
-      cudaGraphNodeParams* cp = reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
-      cp->type = cudaGraphNodeTypeConditional;
-      cp->conditional.handle = h;
-      cp->conditional.type = cudaGraphCondTypeWhile;
-      cp->conditional.size = 1;
-      cudaGraphNode_t cnode;
-      if (e == cudaSuccess) e = cudaGraphAddNode(&cnode, g, &nodes[0], nullptr, 1, cp);
-      if (e == cudaSuccess) {
-        // body: the iteration up to the update decision, then a conditional
-        // node holding the reliable update, entered only when it is due
-        cudaGraph_t body = cp->conditional.phGraph_out[0];
-        cudaGraphConditionalHandle hu = 0;
-        e = cudaGraphConditionalHandleCreate(&hu, body, 0, 0);
-        if (e == cudaSuccess)
-          e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-        cudaGraphNode_t leaf[4];
-        size_t nleaf = 0;
-        if (e == cudaSuccess) {
-          st = launch_iter(ctx, A32, A64, b, x, B, h, hu, 1);
-          cudaStreamCaptureStatus cs;
-          const cudaGraphNode_t* deps = nullptr;
-          size_t nd = 0;
-          cudaError_t e1 = cudaStreamGetCaptureInfo(s, &cs, nullptr, nullptr, &deps, nullptr, &nd);
-          if (e1 == cudaSuccess && nd >= 1 && nd <= 4) {
-            for (size_t i = 0; i < nd; ++i) leaf[i] = deps[i];
-            nleaf = nd;
-          } else if (e1 == cudaSuccess) {
-            e1 = cudaErrorUnknown;
-          }
-          cudaGraph_t tmp;
-          cudaError_t e2 = cudaStreamEndCapture(s, &tmp);
-          if (e == cudaSuccess) e = e1;
-          if (e == cudaSuccess) e = e2;
-        }
-        alignas(cudaGraphNodeParams) unsigned char up_buf[sizeof(cudaGraphNodeParams)];
-        memset(up_buf, 0, sizeof(up_buf));
-        cudaGraphNodeParams* up = reinterpret_cast<cudaGraphNodeParams*>(up_buf);
-        up->type = cudaGraphNodeTypeConditional;
-        up->conditional.handle = hu;
-        up->conditional.type = cudaGraphCondTypeIf;
-        up->conditional.size = 1;
-        cudaGraphNode_t unode;
-        if (e == cudaSuccess && st == MFE_OK) e = cudaGraphAddNode(&unode, body, leaf, nullptr, nleaf, up);
-        if (e == cudaSuccess && st == MFE_OK) {
-          cudaGraph_t ubody = up->conditional.phGraph_out[0];
-          e = cudaStreamBeginCaptureToGraph(s, ubody, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-          if (e == cudaSuccess) {
-            st = launch_update(ctx, A64, b, x, B, h, 1);
-            cudaGraph_t tmp;
-            cudaError_t e2 = cudaStreamEndCapture(s, &tmp);
-            if (e == cudaSuccess) e = e2;
-          }
-        }
-      }
-      ctx->stream = run_stream;
-      if (e == cudaSuccess && st == MFE_OK) e = cudaGraphInstantiate(&ex, g, 0);
-      if (e == cudaSuccess && st == MFE_OK) e = cudaGraphLaunch(ex, ctx->stream);
-    }
-    if (ex) cudaGraphExecDestroy(ex);
-    if (g) cudaGraphDestroy(g);
-    if (st != MFE_OK) return st;
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "mixed CG graph");
+    GraphLoop L;
+    L.begin = [&](cudaGraphConditionalHandle h) {
+      k_mx_begin<<<1, 1, 0, ctx->stream>>>(B.st, h);
+      return check_launch(ctx, "k_mx_begin");
+    };
+    // the iteration up to the update decision; the reliable update in a
+    // conditional node, entered only when it is due
+    L.body = [&](cudaGraphConditionalHandle h, cudaGraphConditionalHandle hu) {
+      return launch_iter(ctx, A32, A64, b, x, B, h, hu, 1);
+    };
+    L.update = [&](cudaGraphConditionalHandle h) { return launch_update(ctx, A64, b, x, B, h, 1); };
+    L.copies = B.stencil ? kCopies : 1;
+    MFE_TRY(run_graph_loop(ctx, L, "mixed CG graph"));
   }
   MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, B.st, sizeof(MixState), cudaMemcpyDeviceToHost, ctx->stream));
   MFE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, ctx->stream));

@@ -80,6 +80,7 @@ struct MultiState {
   int done[kMaxRhs];
   int iters[kMaxRhs];  // iterations until each right-hand side converged
   int brk[kMaxRhs];    // p.Ap <= 0 met (the right-hand side stops alone)
+  int run;  // 0: the rest of the loop body's iterations do nothing
   int nrhs, k, max_iter, since, refine_k, gate, cont, first, updates, status, tol_mode;
   int max_refine;  // mixed: stop after this many shared updates (0: no cap)
   unsigned err;
@@ -820,6 +821,7 @@ __global__ void __launch_bounds__(kSMW * 32) k_spmm_st32(const __grid_constant__
   constexpr unsigned kAll = (1u << (3 * W)) - 1u;
   __shared__ double red[kSMW * 32];
   const int warp = threadIdx.x >> 5;
+  if (P.st->run == 0) return;
   const int64_t items = (int64_t)P.nzc * P.ntile;
   DFAcc facc;
   for (int64_t it = (int64_t)blockIdx.x * kSMW + warp; it < items; it += (int64_t)gridDim.x * kSMW) {
@@ -911,6 +913,7 @@ __global__ void __launch_bounds__(kVT)
   constexpr int VW = Vec16<V>::n;
   const int64_t g0 = (int64_t)blockIdx.x * kVT + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * kVT;
+  if (st->run == 0) return;
   const bool first = st->first != 0;
   // mixed (V = float): the last update's x32 += alpha p, done here where the
   // old p is read anyway (st->alpha still holds that update's alphas), unless
@@ -973,6 +976,7 @@ __global__ void __launch_bounds__(kVT)
   __shared__ double ent[kVT * VW];
   const int64_t g0 = (int64_t)blockIdx.x * kVT + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * kVT;
+  if (st->run == 0) return;
   V alpha[VW];
 #pragma unroll
   for (int c = 0; c < VW; ++c) {
@@ -1062,6 +1066,7 @@ __global__ void __launch_bounds__(kVT)
 __global__ void k_mr_decide(MultiState* st, cudaGraphConditionalHandle h_loop,
                             cudaGraphConditionalHandle h_upd, int in_graph)
 {
+  if (st->run == 0) return;
   const int j = threadIdx.x;
   const int nr = st->nrhs;
   bool ready = true, brk = false;
@@ -1097,7 +1102,10 @@ __global__ void k_mr_decide(MultiState* st, cudaGraphConditionalHandle h_loop,
       cudaGraphSetConditional(h_loop, st->cont ? 1u : 0u);
     }
   }
-  if (j == 0) cudaGraphSetConditional(h_upd, gate ? 1u : 0u);
+  if (j == 0) {
+    st->run = !gate && st->cont;
+    cudaGraphSetConditional(h_upd, gate ? 1u : 0u);
+  }
 }
 
 // Mixed solver, one warp, after the gated FP64 residual: per right-hand side
@@ -1136,6 +1144,7 @@ __global__ void k_mr_after(MultiState* st, cudaGraphConditionalHandle h, int in_
     st->gate = 0;
     st->cont = open && st->k < st->max_iter &&
                !(gate && st->max_refine > 0 && st->updates >= st->max_refine);
+    st->run = st->cont;
     if (in_graph) cudaGraphSetConditional(h, st->cont ? 1u : 0u);
   }
 }
@@ -1190,7 +1199,7 @@ __global__ void k_mr_init(MultiState* st)
     st->iters[j] = 0;
   }
   const bool open = __any_sync(0xffffffffu, j < nr && !st->done[j]);
-  if (j == 0) st->cont = open && st->max_iter > 0;
+  if (j == 0) st->run = st->cont = open && st->max_iter > 0;
 }
 
 __global__ void k_mr_begin(const MultiState* st, cudaGraphConditionalHandle h)
@@ -1436,7 +1445,7 @@ mfe_status multi_iter_f64(mfe_ctx* ctx, const mfe_csr& A64, int nrhs, double* X,
 // condition set by the body (the handle passed as body's second argument).
 template <typename Body, typename Update>
 mfe_status run_loop(mfe_ctx* ctx, MultiState* dev_st, MultiState* host_st, Body body,
-                    Update update, bool with_update)
+                    Update update, bool with_update, int copies)
 {
   if (getenv("MFE_CG_EAGER") != nullptr) {
     for (;;) {
@@ -1448,92 +1457,15 @@ mfe_status run_loop(mfe_ctx* ctx, MultiState* dev_st, MultiState* host_st, Body 
       if (with_update) MFE_TRY(update((cudaGraphConditionalHandle)0, 0));
     }
   }
-  cudaStream_t run_stream = ctx->stream, s = ctx->own_stream;
-  cudaGraph_t g = nullptr;
-  cudaGraphExec_t ex = nullptr;
-  cudaGraphConditionalHandle h = 0;
-  mfe_status st = MFE_OK;
-  cudaError_t e = cudaGraphCreate(&g, 0);
-  if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-  if (e == cudaSuccess) {
-    ctx->stream = s;
-    e = cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-    if (e == cudaSuccess) {
-      k_mr_begin<<<1, 1, 0, s>>>(dev_st, h);
-      e = cudaStreamEndCapture(s, &g);
-    }
-    cudaGraphNode_t nodes[4];
-    size_t nn = 4;
-    if (e == cudaSuccess) e = cudaGraphGetNodes(g, nodes, &nn);
-    alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)];
-    memset(cp_buf, 0, sizeof(cp_buf));
-    cudaGraphNodeParams* cp = reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
-    cp->type = cudaGraphNodeTypeConditional;
-    cp->conditional.handle = h;
-    cp->conditional.type = cudaGraphCondTypeWhile;
-    cp->conditional.size = 1;
-    cudaGraphNode_t cnode;
-    if (e == cudaSuccess) e = cudaGraphAddNode(&cnode, g, &nodes[0], nullptr, 1, cp);
-    if (e == cudaSuccess) {
-      cudaGraph_t body_graph = cp->conditional.phGraph_out[0];
-      cudaGraphConditionalHandle hu = 0;
-      if (with_update) e = cudaGraphConditionalHandleCreate(&hu, body_graph, 0, 0);
-      if (e == cudaSuccess)
-        e = cudaStreamBeginCaptureToGraph(s, body_graph, nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeRelaxed);
-      cudaGraphNode_t leaf[4];
-      size_t nleaf = 0;
-      if (e == cudaSuccess) {
-        st = body(h, hu, 1);
-        cudaError_t e1 = cudaSuccess;
-        if (with_update) {
-          cudaStreamCaptureStatus cs;
-          const cudaGraphNode_t* deps = nullptr;
-          size_t nd = 0;
-          e1 = cudaStreamGetCaptureInfo(s, &cs, nullptr, nullptr, &deps, nullptr, &nd);
-          if (e1 == cudaSuccess && nd >= 1 && nd <= 4) {
-            for (size_t i = 0; i < nd; ++i) leaf[i] = deps[i];
-            nleaf = nd;
-          } else if (e1 == cudaSuccess) {
-            e1 = cudaErrorUnknown;
-          }
-        }
-        cudaGraph_t tmp;
-        const cudaError_t e2 = cudaStreamEndCapture(s, &tmp);
-        if (e == cudaSuccess) e = e1;
-        if (e == cudaSuccess) e = e2;
-      }
-      if (with_update && e == cudaSuccess && st == MFE_OK) {
-        alignas(cudaGraphNodeParams) unsigned char up_buf[sizeof(cudaGraphNodeParams)];
-        memset(up_buf, 0, sizeof(up_buf));
-        cudaGraphNodeParams* up = reinterpret_cast<cudaGraphNodeParams*>(up_buf);
-        up->type = cudaGraphNodeTypeConditional;
-        up->conditional.handle = hu;
-        up->conditional.type = cudaGraphCondTypeIf;
-        up->conditional.size = 1;
-        cudaGraphNode_t unode;
-        e = cudaGraphAddNode(&unode, body_graph, leaf, nullptr, nleaf, up);
-        if (e == cudaSuccess) {
-          e = cudaStreamBeginCaptureToGraph(s, up->conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                            cudaStreamCaptureModeRelaxed);
-          if (e == cudaSuccess) {
-            st = update(h, 1);
-            cudaGraph_t tmp;
-            const cudaError_t e2 = cudaStreamEndCapture(s, &tmp);
-            if (e == cudaSuccess) e = e2;
-          }
-        }
-      }
-    }
-    ctx->stream = run_stream;
-    if (e == cudaSuccess && st == MFE_OK) e = cudaGraphInstantiate(&ex, g, 0);
-    if (e == cudaSuccess && st == MFE_OK) e = cudaGraphLaunch(ex, ctx->stream);
-  }
-  if (ex) cudaGraphExecDestroy(ex);
-  if (g) cudaGraphDestroy(g);
-  if (st != MFE_OK) return st;
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "multi-RHS CG graph");
-  return MFE_OK;
+  GraphLoop L;
+  L.begin = [&](cudaGraphConditionalHandle h) {
+    k_mr_begin<<<1, 1, 0, ctx->stream>>>(dev_st, h);
+    return check_launch(ctx, "k_mr_begin");
+  };
+  L.body = [&](cudaGraphConditionalHandle h, cudaGraphConditionalHandle hu) { return body(h, hu, 1); };
+  if (with_update) L.update = [&](cudaGraphConditionalHandle h) { return update(h, 1); };
+  L.copies = copies;
+  return run_graph_loop(ctx, L, "multi-RHS CG graph");
 }
 
 }  // namespace
@@ -1711,7 +1643,7 @@ mfe_status cg_multi(mfe_ctx* ctx, const mfe_csr* A64_in, int nrhs, const double*
         [&](cudaGraphConditionalHandle h, int in_graph) {
           return multi_update_mixed(ctx, A64, nrhs, B, X, W, h, in_graph);
         },
-        true));
+        true, use_st32 ? 8 : 1));
   } else {
     MultiBufs<double> W{static_cast<double*>(r), static_cast<double*>(p),
                         static_cast<double*>(Ap), nullptr, dst, partials, tickets, err};
@@ -1720,7 +1652,7 @@ mfe_status cg_multi(mfe_ctx* ctx, const mfe_csr* A64_in, int nrhs, const double*
         [&](cudaGraphConditionalHandle h, cudaGraphConditionalHandle, int in_graph) {
           return multi_iter_f64(ctx, A64, nrhs, X, W, h, in_graph);
         },
-        [&](cudaGraphConditionalHandle, int) { return MFE_OK; }, false));
+        [&](cudaGraphConditionalHandle, int) { return MFE_OK; }, false, 1));
   }
   unsigned* herr = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(hs) + sizeof(MultiState));
   MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, dst, sizeof(MultiState), cudaMemcpyDeviceToHost, ctx->stream));

@@ -187,6 +187,7 @@ struct StParams {
   unsigned* ticket;
   double* dot_out;
   unsigned* err;
+  const int* run;  // when set and *run == 0 the launch does nothing
 };
 
 // first float of the copy of line (z, dy = j - 1) for plane positions
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(kS2P / 2 + 32, kSep ? 3 : 2)
   __shared__ uint64_t full[kSS], empty[kSS];
   __shared__ float2 red[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (P.run != nullptr && *P.run == 0) return;
   const int64_t T = (int64_t)P.ntile * P.Nz;
   const int64_t q0 = T * blockIdx.x / gridDim.x, q1 = T * (blockIdx.x + 1) / gridDim.x;
   if (threadIdx.x == 0) {
@@ -656,9 +658,10 @@ mfe_status stencil_grid(mfe_ctx* ctx, const float* coef, int* grid)
 }
 
 mfe_status launch_spmv_stencil(mfe_ctx* ctx, const mfe_csr* A, const float* coef, const float* x,
-                               float* y, const DotSink* sink, int grid, unsigned* err)
+                               float* y, const DotSink* sink, int grid, unsigned* err, const int* run)
 {
   StParams P;
+  P.run = run;
   P.Nx = A->box_nx + 1;
   P.Ny = A->box_ny + 1;
   P.Nz = A->box_nz + 1;
