@@ -423,6 +423,139 @@ __global__ void __launch_bounds__(kStgWarps * 32, 5) k_spmv_staged(SpmvParams<T>
   }
 }
 
+// FP64 CSR rows whose longest is not known: staged as in k_spmv_staged, with a
+// stage of `cap` entries (the host's guess from the mean row length).  Groups
+// that do not fit it, or hold a row over twice the unrolled length, read from
+// global memory, a row at a time over the warp.  So no pass over the row
+// offsets and no read-back precede the product: 1.48 M rows of 4 to 27 entries
+// 107 us per call against 121.  What bounds it: row_dot's 27 FMAs per row
+// whatever its length (the FP64 pipe is busy two thirds of the time).  Cutting
+// a group's entries into 32 equal runs instead, a lane per run, took a quarter
+// less of the FP64 pipe but twice the instructions, 147 us.
+constexpr int kAnyLongest = 54;
+template <int MODE>
+__global__ void __launch_bounds__(kStgWarps * 32, 5) k_spmv_any(SpmvParams<double> P, int cap)
+{
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint64_t bar[kStgWarps][kStgStages];
+  __shared__ double red[32];
+  const int lane = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5;
+  const size_t vbytes = (size_t)cap * sizeof(double);
+  const size_t sbytes = vbytes + (size_t)cap * sizeof(int32_t);
+  unsigned char* wbase = smem + (size_t)w * kStgStages * sbytes;
+  const int64_t ngroups = (P.n + 31) / 32;
+  const int64_t nw = (int64_t)gridDim.x * kStgWarps;
+  const int64_t g0 = (int64_t)blockIdx.x * kStgWarps + w;
+  if (lane == 0) {
+    for (int s = 0; s < kStgStages; ++s) mbar_init(&bar[w][s], 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+
+  // up to 3 elements of slack at each end of a group (16-byte boundaries)
+  auto staged = [&](int64_t a, int64_t e) { return e - a + 8 <= cap; };
+  // lane 0: nonzeros [a, e) of one group into stage s
+  auto issue = [&](int64_t a, int64_t e, int s) {
+    if (!staged(a, e)) {
+      mbar_arrive_expect_tx(&bar[w][s], 0);
+      return;
+    }
+    const int64_t av = a & ~(int64_t)1, ac = a & ~(int64_t)3;
+    const int64_t bv = max(av, min((e + 1) & ~(int64_t)1, P.nnz & ~(int64_t)1));
+    const int64_t bc = max(ac, min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3));
+    double* dv = reinterpret_cast<double*>(wbase + (size_t)s * sbytes);
+    int32_t* dc = reinterpret_cast<int32_t*>(wbase + (size_t)s * sbytes + vbytes);
+    // ragged tail past the last 16-byte boundary of the arrays: plain loads
+    for (int64_t k = bv; k < e; ++k) dv[k - av] = P.vals[k];
+    for (int64_t k = bc; k < e; ++k) dc[k - ac] = P.cols[k];
+    fence_proxy_async_smem();
+    const unsigned bytes_v = (unsigned)((bv - av) * sizeof(double));
+    const unsigned bytes_c = (unsigned)((bc - ac) * sizeof(int32_t));
+    mbar_arrive_expect_tx(&bar[w][s], bytes_v + bytes_c);
+    if (bytes_v) bulk_g2s(dv, P.vals + av, bytes_v, &bar[w][s]);
+    if (bytes_c) bulk_g2s(dc, P.cols + ac, bytes_c, &bar[w][s]);
+  };
+  auto bounds = [&](int64_t g, int64_t& a, int64_t& e) {
+    a = __ldg(&P.ro[g * 32]);
+    e = __ldg(&P.ro[min(P.n, g * 32 + 32)]);
+  };
+
+  if (lane == 0 && P.withhold_ns == 0)
+    for (int s = 0; s < kStgStages; ++s) {
+      const int64_t g = g0 + (int64_t)s * nw;
+      int64_t a, e;
+      if (g < ngroups) {
+        bounds(g, a, e);
+        issue(a, e, s);
+      }
+    }
+  const uint64_t wait_ns = P.withhold_ns ? P.withhold_ns : kWaitLimitNs;
+  double dacc = 0.0;
+  bool ok = true;
+  int it = 0;
+  for (int64_t g = g0; g < ngroups; g += nw, ++it) {
+    const int s = it % kStgStages;
+    const int64_t r = g * 32 + lane;
+    const int64_t gn = g + (int64_t)kStgStages * nw;  // the group stage s takes next
+    int64_t a, e, na = 0, ne = 0;
+    bounds(g, a, e);
+    const int m = (int)(e - a);
+    int st = m, en = m;  // the lane's row, from a
+    if (r < P.n) {
+      st = (int)(__ldg(&P.ro[r]) - a);
+      en = (int)(__ldg(&P.ro[r + 1]) - a);
+    }
+    if (lane == 0 && gn < ngroups) bounds(gn, na, ne);
+    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w][s], (unsigned)((it / kStgStages) & 1), wait_ns));
+    if (!ok) break;
+    double sum = 0.0;
+    if (staged(a, e) && __reduce_max_sync(0xffffffffu, en - st) <= kAnyLongest) {
+      const double* gv = reinterpret_cast<const double*>(wbase + (size_t)s * sbytes) + (a & 1);
+      const int32_t* gc = reinterpret_cast<const int32_t*>(wbase + (size_t)s * sbytes + vbytes) + (a & 3);
+      sum = row_dot<double, 27>(gv + st, gc + st, en - st, P.x);
+    } else {
+      for (int j = 0; j < 32; ++j) {
+        const int js = __shfl_sync(0xffffffffu, st, j), je = __shfl_sync(0xffffffffu, en, j);
+        double v = 0.0;
+        for (int k = js + lane; k < je; k += 32) v = fma(P.vals[a + k], __ldg(&P.x[P.cols[a + k]]), v);
+        v = warp_sum(v);
+        if (lane == j) sum = v;
+      }
+    }
+    if (r < P.n) {
+      if (MODE == SPMV_RESID) {
+        const double rr = P.b[r] - sum;
+        P.y[r] = rr;
+        dacc = fma(rr, rr, dacc);
+      } else {
+        P.y[r] = sum;
+        if (MODE == SPMV_DOT) dacc = fma(sum, __ldg(&P.x[r]), dacc);
+      }
+    }
+    __syncwarp();  // every lane is done reading stage s
+    if (lane == 0 && gn < ngroups) issue(na, ne, s);
+  }
+  if (!ok) {
+    if (lane == 0) {
+      atomicOr(P.err, ERR_WAIT_TIMEOUT);
+      // drain: give each stage with a copy issued a bounded chance to land
+      // before the block exits (an injected fault issued none)
+      for (int j = it; j < it + kStgStages; ++j)
+        if (P.withhold_ns == 0 && g0 + (int64_t)j * nw < ngroups)
+          mbar_wait_bounded(&bar[w][j % kStgStages], (unsigned)((j / kStgStages) & 1));
+    }
+    __syncwarp();
+  }
+  // every warp reaches the block reduction, also after a timeout
+  if (MODE != SPMV_PLAIN) {
+    const double bt = block_sum(dacc, red);
+    double total;
+    if (grid_reduce_last(bt, P.partials, P.ticket, red, &total) && threadIdx.x == 0)
+      spmv_epilogue<MODE>(total, P.cg, P.dot_out);
+  }
+}
+
 // The reference's row-major ELL, K entries per row (K <= kStgMaxLen): group
 // g's entries start at 32 g K, 16-byte aligned in both arrays, and row lane
 // sits at lane K of its stage.  The stage size is computed from K here (not
@@ -723,13 +856,43 @@ static mfe_status launch_staged(mfe_ctx* ctx, SpmvParams<T>& P, int max_len)
   return check_launch(ctx, "k_spmv_staged");
 }
 
+// k_spmv_any for rows of mean length `mean`: the stage holds 1.3 times the
+// mean and two entries more per row, 32 at most (rows of independent lengths
+// hardly ever fill it: 720 of 800 entries at most over 46,000 groups of rows of
+// 4 to 27)
+static int any_cap(double mean) { return stg_cap(std::max(1, std::min(kStgMaxLen, (int)(1.3 * mean) + 2)), false); }
+
+static size_t any_smem(int cap) { return (size_t)kStgWarps * kStgStages * cap * (sizeof(double) + sizeof(int32_t)); }
+
+static int any_grid(mfe_ctx* ctx, int64_t nrows, int cap)
+{
+  const int per_sm = std::max(1, std::min(16, (int)((227 * 1024) / (any_smem(cap) + 3072))));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)kStgWarps),
+                                                     (int64_t)ctx->sm_count * per_sm));
+}
+
+template <int MODE>
+static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<double>& P)
+{
+  static bool configured[64] = {};
+  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<MODE>, any_smem(stg_cap(kStgMaxLen, false)), configured));
+  const int cap = any_cap((double)P.nnz / (double)P.n);
+  MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
+  k_spmv_any<MODE><<<any_grid(ctx, P.n, cap), kStgWarps * 32, any_smem(cap), ctx->stream>>>(P, cap);
+  return check_launch(ctx, "k_spmv_any");
+}
+
 int spmv_grid(mfe_ctx* ctx, const mfe_csr* A)
 {
   const int max_len = A->max_row_len > 0 ? A->max_row_len : kStgMaxLen;
   if (max_len > kStgMaxLen)  // the warp-per-row kernel
     return (int)std::max<int64_t>(
         1, std::min<int64_t>(ceil_div(A->nrows * 32, 256), (int64_t)ctx->sm_count * 8));
-  if (A->dtype == MFE_F64) return staged_grid<double>(ctx, A->nrows, max_len, false);
+  if (A->dtype == MFE_F64) {
+    if (A->max_row_len <= 0)
+      return any_grid(ctx, A->nrows, any_cap((double)A->nnz / std::max<int64_t>(A->nrows, 1)));
+    return staged_grid<double>(ctx, A->nrows, max_len, false);
+  }
   const int rows = tile_rows();
   const int64_t ntiles = ceil_div(A->nrows, rows);
   const int per_sm = tiled_ctas_per_sm(tiled_smem<float>(rows, max_len));
@@ -782,6 +945,7 @@ static mfe_status launch_t(mfe_ctx* ctx, const mfe_csr* A, const T* x, T* y, con
   if (A->nrows == 0) return MFE_OK;
   if (max_len <= kStgMaxLen && aligned16(A->vals) && aligned16(A->cols)) {
     if constexpr (sizeof(T) == 8) {
+      if (max_len <= 0) return launch_any<MODE>(ctx, P);
       return launch_staged<T, MODE>(ctx, P, max_len);
     } else {
       MFE_CUDA_TRY(ctx, configure_tiled(ctx->device));
@@ -811,8 +975,14 @@ mfe_status launch_spmv(mfe_ctx* ctx, const mfe_csr* A, const void* x, void* y,
   if (csr_is_box(A) && aligned16(A->vals) && aligned16(x) &&
       getenv("MFE_SPMV_GENERIC") == nullptr)
     return launch_spmv_box(ctx, A, x, y, sink, resid_b, cg_state);
-  int max_len = 0;
-  MFE_TRY(ensure_max_row_len(ctx, A, &max_len));
+  // the longest row decides the kernel; FP64 rows of a mean length within the
+  // staged kernels' need not have it found first (k_spmv_any)
+  int max_len = A->max_row_len;
+  if (A->dtype == MFE_F64 && max_len <= 0) {
+    if (A->nnz > (int64_t)kStgMaxLen * A->nrows) max_len = kStgMaxLen + 1;
+  } else {
+    MFE_TRY(ensure_max_row_len(ctx, A, &max_len));
+  }
   CgState* cg = static_cast<CgState*>(cg_state);
   if (A->dtype == MFE_F64) {
     const double* xd = static_cast<const double*>(x);
