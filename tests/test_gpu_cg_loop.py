@@ -7,9 +7,11 @@ relative at most) and, for the stencil operator, in how a product is rounded
 1e-15, and so does x, the norms of r and p being within a factor of ten of b's.
 (Further iterations amplify without a simple bound: the Dirichlet rows are an
 eigenspace that CG resolves at once.)  The boxes lie
-on both sides of the lines where the loop changes its block size (38,912 rows
-on 152 SMs), its form of the stencil product (200,000) and gives way to the
-graph (1,000,000 rows with the CSR values, 2,000,000 with the stencil)."""
+on both sides of the lines where the loop (on 152 SMs) changes its block size
+(91,200 rows with the stencil, 212,800 with the CSR values), no longer holds all
+CSR values in shared memory (about 134,000), changes its form of the stencil
+product (500,000) and gives way to the graph (1,000,000 rows with the CSR
+values, 2,000,000 with the stencil)."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -21,7 +23,8 @@ if not torch.cuda.is_available():  # pragma: no cover - CPU-only machines
 import minife_gb300 as M  # noqa: E402
 
 BOXES = [(1, 1, 1), (2, 1, 3), (7, 4, 5), (33, 32, 33), (34, 33, 32), (58, 57, 57), (58, 58, 57),
-         (99, 99, 98), (99, 99, 99), (600, 12, 20)]
+         (44, 44, 44), (45, 44, 44), (50, 50, 50), (51, 51, 50), (60, 58, 58), (61, 58, 58), (78, 78, 79),
+         (79, 79, 79), (99, 99, 98), (99, 99, 99), (600, 12, 20)]
 
 
 def solve(A, b, x, **kw):
