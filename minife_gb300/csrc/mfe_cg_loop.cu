@@ -33,11 +33,10 @@
 // and two five-step sums at 120 clocks a step), seven warps' 27 FMAs on an SM's
 // FP64 pipe 1.7 us; from 64^3 on the FP64 pipe: 32 operations per row with the
 // CSR values, 22 with the stencil.
-#include <atomic>
-
 #include "mfe_box.cuh"
 #include "mfe_cgstate.cuh"
 #include "mfe_fixed64.cuh"
+#include "mfe_gridloop.cuh"
 
 namespace mfe {
 
@@ -60,78 +59,6 @@ struct LoopParams {
   int Nx, Ny, Nz;
   double w[8], dd;         // stencil operator in FP64: class weights, Dirichlet diagonal
 };
-
-// The calling thread's block arrives at a barrier of all blocks and waits;
-// false after the time limit.
-__device__ __forceinline__ bool arrive_and_wait(unsigned* arrived, unsigned target)
-{
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
-  auto there = [&] {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
-    return (int)(v - target) >= 0;
-  };
-  if (there()) return true;
-  const uint64_t t0 = global_ns();
-  for (unsigned i = 1; !there(); ++i)
-    if ((i & 255u) == 0 && global_ns() - t0 > kWaitLimitNs) return false;
-  return true;
-}
-
-// All blocks; false (in every thread of the block) after the time limit.
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target)
-{
-  __shared__ bool s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) s_ok = arrive_and_wait(arrived, target);
-  __syncthreads();
-  return s_ok;
-}
-
-// The sum of v over all threads of all blocks, given to then(total) in thread 0
-// of every block before a block barrier.  The FP64 pipe takes one warp's
-// addition in 17 clocks, so a reduction by shuffles in every warp would cost
-// more than the rest: one warp adds the block's values from shared memory, and
-// after the grid barrier the blocks' sums in block order.  s_v: a double per
-// thread; beside(): what thread 32 does meanwhile.
-template <int NT, typename Then, typename Beside>
-__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, unsigned* arrived, unsigned target,
-                                         Then&& then, Beside&& beside)
-{
-  __shared__ bool s_ok;
-  s_v[threadIdx.x] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int i = 0; i < NT / 32; ++i) a[i & 3] += s_v[i * 32 + threadIdx.x];
-    const double bt = warp_sum((a[0] + a[1]) + (a[2] + a[3]));
-    bool ok = true;
-    if (threadIdx.x == 0) {
-      __stcg(slots + blockIdx.x, bt);
-      ok = arrive_and_wait(arrived, target);
-    }
-    __syncwarp();
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
-    for (unsigned i = threadIdx.x, j = 0; i < gridDim.x; i += 32, ++j) t[j & 3] += __ldcg(slots + i);
-    const double total = warp_sum((t[0] + t[1]) + (t[2] + t[3]));
-    if (threadIdx.x == 0) {
-      s_ok = ok;
-      then(total);
-    }
-  } else if (threadIdx.x == 32) {
-    beside();
-  }
-  __syncthreads();
-  return s_ok;
-}
-
-template <int NT, typename Then>
-__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, unsigned* arrived, unsigned target,
-                                         Then&& then)
-{
-  return grid_sum<NT>(v, s_v, slots, arrived, target, then, [] {});
-}
 
 // row r of the box CSR times p: k_spmv_box's two sums over the 27 slots; vals:
 // the values of the warp's 32 rows, from the first lane's row; taken() when
@@ -216,12 +143,6 @@ __device__ __forceinline__ double stencil_rows(const LoopParams& P, int first, d
   return row ? centre + (l + u) : P.dd * q[4];
 }
 
-// A block's share of the vector updates: an even range of rows.
-__device__ __forceinline__ int64_t share(int64_t n, unsigned b, unsigned nb)
-{
-  return b == nb ? n : (n * b / nb) & ~(int64_t)1;
-}
-
 // product(Ap): the block's rows of Ap (Ap: where the block keeps its own share);
 // returns the thread's terms of p.Ap.  held: the shared memory for P.held vectors.
 template <int NT, typename Op>
@@ -236,8 +157,8 @@ __device__ __forceinline__ void cg_loop(const LoopParams& P, double* held, Op&& 
   if (tid == 0) S = *P.st;
   __syncthreads();
   if (!S.cont || S.check_pending) return;
-  const int64_t c0 = share(P.n, blockIdx.x, G);
-  const int m = (int)(share(P.n, blockIdx.x + 1, G) - c0), h = m / 2;
+  const int64_t c0 = share<2>(P.n, blockIdx.x, G);
+  const int m = (int)(share<2>(P.n, blockIdx.x + 1, G) - c0), h = m / 2;
   const bool tail = (m & 1) && tid == 0;  // an odd n leaves the last block's last entry
   // the share's vectors where the block keeps them, and p where the others read it
   double* const r1 = P.held > 0 ? held : P.r + c0;
@@ -405,7 +326,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_loop_stencil(const __grid_constant__ LoopParams P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int c0 = (int)share(P.n, blockIdx.x, gridDim.x), c1 = (int)share(P.n, blockIdx.x + 1, gridDim.x);
+  const int c0 = (int)share<2>(P.n, blockIdx.x, gridDim.x), c1 = (int)share<2>(P.n, blockIdx.x + 1, gridDim.x);
   cg_loop<NT>(P, reinterpret_cast<double*>(smem), [&](double* Ap) {
     double d = 0.0;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -434,7 +355,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_loop_csr(const __grid_constant__ L
 {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int NW = NT / 32;
-  const int c0 = (int)share(P.n, blockIdx.x, gridDim.x), c1 = (int)share(P.n, blockIdx.x + 1, gridDim.x);
+  const int c0 = (int)share<2>(P.n, blockIdx.x, gridDim.x), c1 = (int)share<2>(P.n, blockIdx.x + 1, gridDim.x);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (c1 - c0 + 31) / 32, held = min(P.held_chunks, chunks);
   double* const hv = reinterpret_cast<double*>(smem) + P.held * P.span;
@@ -495,45 +416,12 @@ __global__ void __launch_bounds__(NT, NB)
   });
 }
 
-// Shared memory for a block's static part and the system's, out of 227 KB per
-// block and 228 KB per SM.
-constexpr size_t kReserved = 8 * 1024;
-
-// How many of its vectors a block can hold in `room` bytes, at most `most`;
-// the bytes they take.
-size_t plan_held(LoopParams& P, int g, size_t room, int most)
-{
-  P.span = (int)((ceil_div(P.n, (int64_t)g) + 3) & ~(int64_t)1);
-  P.held = (int)std::min<size_t>(room / (sizeof(double) * P.span), most);
-  return sizeof(double) * P.span * P.held;
-}
-
-// The attribute set and the occupancy asked for, once per kernel and device; a
-// launch of blocks that would not all be resident is refused.
-template <size_t kMost>
-mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads, int per_sm, size_t smem,
-                       std::atomic<int>* ready, void** args)
-{
-  std::atomic<int>& have = ready[ctx->device & 63];
-  if (have.load(std::memory_order_acquire) == 0) {
-    int blocks = 0;
-    MFE_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
-    MFE_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, kMost));
-    if (blocks < per_sm) return fail(ctx, MFE_NOT_SUPPORTED, "the CG loop kernel does not fit the device");
-    have.store(blocks, std::memory_order_release);
-  }
-  MFE_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream));
-  return MFE_OK;
-}
-
-constexpr size_t kRoom = 227 * 1024 - kReserved;
-
 template <int NT>
 mfe_status run_stencil(mfe_ctx* ctx, LoopParams& P)
 {
   static std::atomic<int> ready[64];
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(P.n, 64), ctx->sm_count));
-  const size_t smem = plan_held(P, g, kRoom, 4);
+  const size_t smem = plan_held(P.n, g, sizeof(double), kRoom, 4, &P.span, &P.held);
   void* args[] = {&P};
   return coop_launch<kRoom>(ctx, (const void*)k_cg_loop_stencil<NT>, g, NT, 1, smem, ready, args);
 }
@@ -545,14 +433,14 @@ mfe_status run_csr(mfe_ctx* ctx, LoopParams& P)
   constexpr size_t kChunkBytes = kChunk * sizeof(double), kBuffers = NT / 32 * kChunkBytes;
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(P.n, 64), ctx->sm_count));
   // all values beside all vectors, or the buffers, then vectors, then values
-  size_t smem = plan_held(P, g, kRoom, 4);
+  size_t smem = plan_held(P.n, g, sizeof(double), kRoom, 4, &P.span, &P.held);
   const int chunks = (P.span + 31) / 32;
   if (chunks > kMostChunks) return fail(ctx, MFE_NOT_SUPPORTED, "the CG loop kernel does not fit the device");
   if (P.held == 4 && smem + chunks * kChunkBytes <= kRoom) {
     P.held_chunks = chunks;
     smem += chunks * kChunkBytes;
   } else {
-    smem = plan_held(P, g, kRoom - kBuffers, 4) + kBuffers;
+    smem = plan_held(P.n, g, sizeof(double), kRoom - kBuffers, 4, &P.span, &P.held) + kBuffers;
     P.held_chunks = (int)((kRoom - smem) / kChunkBytes);
     smem += P.held_chunks * kChunkBytes;
   }
@@ -566,7 +454,7 @@ mfe_status run_fixed(mfe_ctx* ctx, LoopParams& P, FxParams& F, int g)
   static std::atomic<int> ready[64];
   constexpr size_t kSweep = FxShape<NT, CM, SEG>::kSmem, kRoom = 227 * 1024 / NB - kReserved;
   static_assert(kSweep <= kRoom, "the sweep's planes");
-  const size_t smem = kSweep + plan_held(P, g, kRoom - kSweep, 3);
+  const size_t smem = kSweep + plan_held(P.n, g, sizeof(double), kRoom - kSweep, 3, &P.span, &P.held);
   void* args[] = {&P, &F};
   return coop_launch<kRoom>(ctx, (const void*)k_cg_loop_fixed<NT, CM, NB, SEG>, g, NT, NB, smem, ready, args);
 }

@@ -1,0 +1,124 @@
+// A solver's iteration loop as one cooperative kernel: barriers and sums over all
+// its blocks, the rows that a block keeps, its launch.  Every wait is bounded.
+#pragma once
+
+#include <algorithm>
+#include <atomic>
+
+#include "mfe_common.cuh"
+#include "mfe_internal.h"
+
+namespace mfe {
+
+// The calling thread's block arrives at a barrier of all blocks and waits;
+// false after the time limit.
+__device__ __forceinline__ bool arrive_and_wait(unsigned* arrived, unsigned target)
+{
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+  auto there = [&] {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+    return (int)(v - target) >= 0;
+  };
+  if (there()) return true;
+  const uint64_t t0 = global_ns();
+  for (unsigned i = 1; !there(); ++i)
+    if ((i & 255u) == 0 && global_ns() - t0 > kWaitLimitNs) return false;
+  return true;
+}
+
+// All blocks; false (in every thread of the block) after the time limit.
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target)
+{
+  __shared__ bool s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) s_ok = arrive_and_wait(arrived, target);
+  __syncthreads();
+  return s_ok;
+}
+
+// The sum of v over all threads of all blocks, given to then(total) in thread 0
+// of every block before a block barrier.  The FP64 pipe takes one warp's
+// addition in 17 clocks, so a reduction by shuffles in every warp would cost
+// more than the rest: one warp adds the block's values from shared memory, and
+// after the grid barrier the blocks' sums in block order.  s_v: a double per
+// thread; beside(): what thread 32 does meanwhile.
+template <int NT, typename Then, typename Beside>
+__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, unsigned* arrived, unsigned target,
+                                         Then&& then, Beside&& beside)
+{
+  __shared__ bool s_ok;
+  s_v[threadIdx.x] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < NT / 32; ++i) a[i & 3] += s_v[i * 32 + threadIdx.x];
+    const double bt = warp_sum((a[0] + a[1]) + (a[2] + a[3]));
+    bool ok = true;
+    if (threadIdx.x == 0) {
+      __stcg(slots + blockIdx.x, bt);
+      ok = arrive_and_wait(arrived, target);
+    }
+    __syncwarp();
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (unsigned i = threadIdx.x, j = 0; i < gridDim.x; i += 32, ++j) t[j & 3] += __ldcg(slots + i);
+    const double total = warp_sum((t[0] + t[1]) + (t[2] + t[3]));
+    if (threadIdx.x == 0) {
+      s_ok = ok;
+      then(total);
+    }
+  } else if (threadIdx.x == 32) {
+    beside();
+  }
+  __syncthreads();
+  return s_ok;
+}
+
+template <int NT, typename Then>
+__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, unsigned* arrived, unsigned target,
+                                         Then&& then)
+{
+  return grid_sum<NT>(v, s_v, slots, arrived, target, then, [] {});
+}
+
+// A block's share of the vectors: a range that begins at a multiple of A (a
+// power of two).
+template <int A>
+__device__ __forceinline__ int64_t share(int64_t n, unsigned b, unsigned nb)
+{
+  return b == nb ? n : (n * b / nb) & ~(int64_t)(A - 1);
+}
+
+// Shared memory for a block's static part and the system's, out of 227 KB per
+// block and 228 KB per SM.
+constexpr size_t kReserved = 8 * 1024, kRoom = 227 * 1024 - kReserved;
+
+// How many of its vectors (n elements of elem bytes over g blocks) a block can
+// hold in `room` bytes, at most `most`; the bytes they take.
+inline size_t plan_held(int64_t n, int g, size_t elem, size_t room, int most, int* span, int* held)
+{
+  *span = (int)((ceil_div(n, (int64_t)g) + 7) & ~(int64_t)3);
+  *held = (int)std::min<size_t>(room / (elem * *span), most);
+  return elem * *span * *held;
+}
+
+// The attribute set and the occupancy asked for, once per kernel and device; a
+// launch of blocks that would not all be resident is refused.
+template <size_t kMost>
+inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads, int per_sm, size_t smem,
+                       std::atomic<int>* ready, void** args)
+{
+  std::atomic<int>& have = ready[ctx->device & 63];
+  if (have.load(std::memory_order_acquire) == 0) {
+    int blocks = 0;
+    MFE_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+    MFE_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, kMost));
+    if (blocks < per_sm) return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
+    have.store(blocks, std::memory_order_release);
+  }
+  MFE_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream));
+  return MFE_OK;
+}
+
+}  // namespace mfe

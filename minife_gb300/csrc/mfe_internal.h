@@ -221,6 +221,13 @@ struct CgLoopArgs {
 };
 mfe_status launch_cg_loop(mfe_ctx* ctx, const mfe_csr* A, const CgLoopArgs& a);
 
+// ---- mixed-precision CG in one cooperative kernel (mfe_mixed_loop.cu) ----
+// FP32 iterations with the mirror-symmetric stencil coef until a reliable update
+// is due or the solve ends; st is the MixState, p has stencil_ghost zero rows
+// on both sides, the vectors are x-padded.
+mfe_status launch_mixed_loop(mfe_ctx* ctx, const mfe_csr* A, const float* coef, float* r, float* p, float* x32,
+                             float* Ap, void* st);
+
 // ---- mixed-precision CG (mfe_mixed.cu) ----
 // Reliable-update policy options of the mixed solvers: an update is due once
 // the recursive residual has fallen by inner_tol since the last one (0: 0.01,

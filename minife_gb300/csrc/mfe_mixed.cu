@@ -24,7 +24,9 @@
 // due (the graph cannot branch cheaply per iteration, so k_mx_xupdate and the
 // FP64 residual SpMV check a device-side gate and return at once when it is
 // closed) and a one-thread bookkeeping kernel that sets the loop condition.
-// The whole solve is one CUDA graph launch with a conditional while node.
+// The whole solve is one CUDA graph launch with a conditional while node; small
+// boxes on the stencil run the iterations up to a reliable update in one
+// cooperative kernel instead (mfe_mixed_loop.cu).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -33,42 +35,19 @@
 
 #include "mfe_common.cuh"
 #include "mfe_internal.h"
+#include "mfe_mixstate.cuh"
 
 namespace mfe {
-
-struct MixState {
-  double rr;            // r.r of the current recursive residual (FP64 accumulated)
-  double rr_new;        // r.r after this iteration's update
-  double pAp;           // written by the FP32 SpMV's epilogue
-  double beta;
-  double rr_true;       // ||b - A x||^2 from the gated FP64 residual SpMV
-  double rr_at_update;  // rr right after the last reliable update
-  double normr0, tol_abs, normr_true;
-  double delta2;        // update when rr_new < delta2 * rr_at_update
-  double alpha_prev;    // alpha of the last update, whose x32 += alpha p is still pending
-  int k;                // inner iterations done
-  int max_iter;
-  int since;            // iterations since the last reliable update
-  int refine_k;         // update at least every refine_k iterations
-  int max_refine;       // stop after this many updates (0: no cap)
-  int gate;             // 1: a reliable update runs in this iteration
-  int cont;             // loop condition
-  int run;              // 0: the rest of the loop body's iterations do nothing
-  int first;            // next p update is p = r
-  int updates;          // reliable updates done
-  int status;           // 0 ok, MFE_BREAKDOWN
-  int record;
-  unsigned err;
-  int x_pending;        // 1: x32 += alpha_prev p is due (done by the next p update or
-                        // the gated x update, whichever comes first)
-  double* history;      // recursive normr per iteration (record)
-};
 
 constexpr int kT = 256;
 constexpr int kMaxPart = 8192;
 // iterations in a row in the loop's body (160 x 192 x 144, us per iteration: 1
 // 46.5, 2 43.5, 4 41.6, 8 40.9; 40^3: 22.7, 19.7, 18.1, 17.6)
 constexpr int kCopies = 8;
+// up to here the iterations between two reliable updates run in one kernel
+// (mfe_mixed_loop.cu: 124^3 27.7 us per iteration against 29.1 here, 160 x 192 x
+// 144 50 against 40.5)
+constexpr int64_t kLoopRows = 2000000;
 
 // p = r (first) or p = r + beta p, FP32 (cg_solve.hpp:153-161).  The previous
 // iteration's x32 += alpha p (cg_solve.hpp:201-205) is done here, where the
@@ -433,12 +412,16 @@ mfe_status cg_mixed(mfe_ctx* ctx, const mfe_csr* A64_in, const double* b, double
   grid_for(ctx, 1, (const void*)k_mx_p);
   grid_for(ctx, 1, (const void*)k_mx_update);
   grid_for(ctx, 1, (const void*)k_mx_xupdate);
-  if (getenv("MFE_CG_EAGER") != nullptr) {
+  const bool eager = getenv("MFE_CG_EAGER") != nullptr;
+  float w8[8];
+  const bool loop = !eager && B.stencil && n <= kLoopRows && stencil_mirror_classes(B.coef, w8);
+  if (eager || loop) {
     for (;;) {
       MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, B.st, sizeof(MixState), cudaMemcpyDeviceToHost, ctx->stream));
       MFE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
       if (!hs->cont || hs->err) break;
-      MFE_TRY(launch_iter(ctx, A32, A64, b, x, B, 0, 0, 0));
+      if (loop) MFE_TRY(launch_mixed_loop(ctx, &A64, B.coef, B.r, B.p, B.x32, B.Ap, B.st));
+      else MFE_TRY(launch_iter(ctx, A32, A64, b, x, B, 0, 0, 0));
       MFE_TRY(launch_update(ctx, A64, b, x, B, 0, 0));
     }
   } else {
