@@ -432,11 +432,13 @@ inline void fx_tiles(FxParams& P, int NT, bool three)
 // CTAs, or as equal runs of one tile's planes each.  A run stages two planes
 // more than it has steps, and an even share may end one tile and begin the
 // next, which costs two planes again, so the choice is the one whose busiest
-// CTA stages the fewest planes, and the larger tile (whose window overlaps its
-// neighbours' less) where they tie.  Measured per iteration in the CG loop, even
-// shares only against this rule: 97 x 64 x 83 elements 36.8 / 33.0 us, 128^3
-// 77.6 / 72.1 us.  The window is one run of positions while the lines between
-// leave it within six elements per thread, else three line segments (node lines
+// CTA stages the fewest planes, and two CTAs per SM where they tie (one computes
+// while the other waits at its plane's barrier, which gains more than the
+// larger tile's smaller overlap).  Measured per iteration: even shares only
+// against this rule, 97 x 64 x 83 elements 36.8 / 33.0 us, 128^3 77.6 / 72.1;
+// one CTA against two at a tie, 150 x 160 x 170 125.5 / 119.2, 200^3 220.6 /
+// 212.3, 240^3 350 / 333, 256^3 417 / 405.  The window is one run of positions
+// while it fits six elements per thread, else three line segments (node lines
 // over 511 long).
 enum FxKind { FX_512 = 0, FX_256X2 = 1, FX_SEG = 2 };
 
@@ -465,10 +467,10 @@ inline FxKind fx_setup(const mfe_ctx* ctx, const mfe_csr* A, const double* w8, d
   fx_tiles(P, 512, false);
   const int64_t p512 = share(ctx->sm_count);
   fx_tiles(P, 256, false);
-  if (2 * P.Nx + 2 <= 2 * 256 && share(2 * ctx->sm_count) < p512) return FX_256X2;
+  if (P.L <= 6 * 256 && share(2 * ctx->sm_count) <= p512) return FX_256X2;
   fx_tiles(P, 512, false);
   share(ctx->sm_count);
-  if (2 * P.Nx + 2 <= 2 * 512) return FX_512;
+  if (P.L <= 6 * 512) return FX_512;
   fx_tiles(P, 256, true);
   share(ctx->sm_count);
   return FX_SEG;
