@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(kVT)
   using VV = typename Vec16<V>::type;
   constexpr int VW = Vec16<V>::n;
   __shared__ double red[(kVT / 32 + 1) * 32];
-  __shared__ double ent[kVT * VW];
+  __shared__ typename std::conditional<sizeof(V) == 4, float2, double>::type ent[kVT * VW];
   const int64_t g0 = (int64_t)blockIdx.x * kVT + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * kVT;
   if (st->run == 0) return;
@@ -1027,13 +1027,25 @@ __global__ void __launch_bounds__(kVT)
     }
   }
   // entry VW*t + c holds right-hand side (VW*t + c) % nrhs; entries t + k*kVT
-  // share thread t's right-hand side t % nrhs
-#pragma unroll
-  for (int c = 0; c < VW; ++c) ent[VW * threadIdx.x + c] = acc[c] + facc[c].value();
-  __syncthreads();
+  // share thread t's right-hand side t % nrhs.  The double-float sums stay so
+  // until one number per thread is left: eleven FP64 additions per thread here
+  // cost a 64^3 x 32 solve 2.2 us per iteration.
   double a = 0.0;
+  if constexpr (sizeof(V) == 4) {
 #pragma unroll
-  for (int k = 0; k < VW; ++k) a += ent[threadIdx.x + k * kVT];
+    for (int c = 0; c < VW; ++c) ent[VW * threadIdx.x + c] = make_float2(facc[c].hi, facc[c].lo);
+    __syncthreads();
+    DFAcc t;
+#pragma unroll
+    for (int k = 0; k < VW; ++k) df_add(t.hi, t.lo, ent[threadIdx.x + k * kVT].x, ent[threadIdx.x + k * kVT].y);
+    a = t.value();
+  } else {
+#pragma unroll
+    for (int c = 0; c < VW; ++c) ent[VW * threadIdx.x + c] = acc[c];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < VW; ++k) a += ent[threadIdx.x + k * kVT];
+  }
   a = lane_group_sum(a, nrhs);
   if ((threadIdx.x & 31) >= nrhs) a = 0.0;
   multi_dot_reduce(a, red, partials, ticket, st->rr_new, nrhs);
