@@ -279,15 +279,11 @@ __global__ void __launch_bounds__(ROWS, 2) k_spmv_tiled(SpmvParams<T> P)
 // contiguous in both layouts below (CSR: ro[32g] .. ro[32g+32]; the
 // reference's ELLMatrix: 32 g K .. 32 (g+1) K, short rows padded).  Lane 0
 // stages a group's values and columns with two 1-D bulk copies (TMA) into the
-// warp's own ring of kStgStages shared-memory stages, each with its mbarrier
-// (no block barrier in the loop), and every lane sums its own row from shared
-// memory with row_dot.  With rows of 27 entries an FP64 stage is 10.5 KB and
-// ten warps per SM each keep their next group in flight, where the tiled
-// kernel's 128-row tiles hold two blocks per SM behind block barriers: the
-// 256^3 FP64 product takes 1.14 ms against 2.09 ms through the tiled kernel
-// (FP32 rows, half the bytes per stage, stay on the tiled kernel: 0.638
-// ms, where the staged form took 0.75-0.80 ms before either kernel stated
-// its blocks per SM).
+// warp's own shared memory, with its own mbarrier (no block barrier in the
+// loop), and every lane sums rows from there.  The 256^3 FP64 CSR product took
+// 1.14 ms this way, two stages per warp, against 2.09 ms with 128-row tiles
+// behind block barriers (FP32 rows, half the bytes per stage, stay on the tiled
+// kernel).
 constexpr int kStgWarps = 2;    // warps per block
 constexpr int kStgStages = 2;   // stages per warp
 constexpr int kStgMaxLen = 32;  // longer rows: the warp-per-row kernel
@@ -301,203 +297,154 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
   return ell ? 32 * max_len : ((32 * max_len + 8) + 3) & ~3;
 }
 
-// CSR rows of at most max_len entries.  A stage starts on the 16-byte
-// boundaries at or below its group's first nonzero, and the ragged end of
-// the arrays arrives by plain loads, as in the tiled kernel.
-// Five blocks per SM is the occupancy shared memory allows for 27-entry rows;
-// stating it (any minimum does) lets ptxas keep a row's gathers in flight at
-// 72 registers instead of 40: 1.14-1.16 against 1.40 ms for the 256^3 product
-template <typename T, int MODE>
-__global__ void __launch_bounds__(kStgWarps * 32, 5) k_spmv_staged(SpmvParams<T> P, int max_len)
+// FP64 CSR rows.  A stage starts on the 16-byte boundaries at or below its
+// group's first nonzero, and the ragged end of the arrays arrives by plain
+// loads.  The stage is one per warp, of `cap` entries (the host's guess from the
+// mean row length): twenty-four warps per SM, a part of them computing while the
+// others' next groups arrive.  Groups that do not fit the stage, or hold a row
+// over kAnyLongest, read from global memory, a row at a time over the warp, so
+// the longest row need not be known.
+//
+// What bounds it: the FP64 pipe, whose instructions take 17 clocks an SM whatever
+// the number of lanes at work.  Hence the rows in pairs (row_pair): 1.48 M rows
+// of 4 to 27 entries, 15.5 on average, take 18 FMAs a group instead of 27.
+// Measured there, us per call: a pass for the longest row, two stages and 27
+// FMAs 121; without the pass 107; in pairs 103; one stage, 8 / 10 / 12 blocks per
+// SM 86 / 79 / 76 (50 are the bytes at the HBM rate).  Rows of 27 entries (no
+// pairs): 126 / 106; of 3 to 7: 120 / 58; of 20 to 40: 682 / 273.  Cutting a
+// group's entries into 32 equal runs, a lane per run, took twice the
+// instructions, 147 us.
+constexpr int kAnyLongest = 54;
+constexpr int kAnyBlocks = 12;  // per SM
+
+// A group's 32 rows shared out in pairs: the lanes ranked by row length, the
+// r-th shortest row's lane also takes the end of the r-th longest, so that both
+// have half of the two rows' entries.  At most kPairSteps entries per lane.
+constexpr int kPairSteps = 18;
+struct RowPair {
+  int other;   // the other row's lane
+  int own;     // entries of the lane's own row that it takes
+  int extra;   // and of the other's, from its entry `from` on
+  int from;
+};
+__device__ __forceinline__ RowPair row_pair(int st, int en, uint8_t* lane_of_rank)
 {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t bar[kStgWarps][kStgStages];
-  __shared__ double red[32];
-  constexpr int VA = 16 / sizeof(T);  // values per 16 bytes
-  const int lane = threadIdx.x & 31;
-  const int w = threadIdx.x >> 5;
-  const int cap = stg_cap(max_len, false);
-  const size_t vbytes = (size_t)cap * sizeof(T);
-  const size_t sbytes = vbytes + (size_t)cap * sizeof(int32_t);
-  unsigned char* wbase = smem + (size_t)w * kStgStages * sbytes;
-  const int64_t ngroups = (P.n + 31) / 32;
-  const int64_t nw = (int64_t)gridDim.x * kStgWarps;
-  const int64_t g0 = (int64_t)blockIdx.x * kStgWarps + w;
-  if (lane == 0) {
-    for (int s = 0; s < kStgStages; ++s) mbar_init(&bar[w][s], 1);
-    fence_mbar_init();
+  const int lane = threadIdx.x & 31, len = en - st;
+  unsigned same = 0xffffffffu;
+  int rank = 0;
+#pragma unroll
+  for (int b = 5; b >= 0; --b) {  // len <= kAnyLongest < 64
+    const bool one = (len >> b) & 1;
+    const unsigned ones = __ballot_sync(0xffffffffu, one);
+    if (one) rank += __popc(same & ~ones);
+    same &= one ? ones : ~ones;
   }
-  __syncthreads();
-
-  // lane 0: nonzeros [a, e) of one group into stage s
-  auto issue = [&](int64_t a, int64_t e, int s) {
-    const int64_t av = a & ~(int64_t)(VA - 1);
-    const int64_t ac = a & ~(int64_t)3;
-    int64_t bv = min((e + VA - 1) & ~(int64_t)(VA - 1), P.nnz & ~(int64_t)(VA - 1));
-    int64_t bc = min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3);
-    if (bv < av) bv = av;
-    if (bc < ac) bc = ac;
-    if (max(bv, e) - av > cap || max(bc, e) - ac > cap) {
-      // cannot happen when every row has <= the max_len the host passed;
-      // record it and stage nothing
-      atomicOr(P.err, ERR_TILE_OVERFLOW);
-      mbar_arrive_expect_tx(&bar[w][s], 0);
-      return;
-    }
-    T* dv = reinterpret_cast<T*>(wbase + (size_t)s * sbytes);
-    int32_t* dc = reinterpret_cast<int32_t*>(wbase + (size_t)s * sbytes + vbytes);
-    // ragged tail past the last 16-byte boundary of the arrays: plain loads
-    for (int64_t k = bv; k < e; ++k) dv[k - av] = P.vals[k];
-    for (int64_t k = bc; k < e; ++k) dc[k - ac] = P.cols[k];
-    fence_proxy_async_smem();
-    const unsigned bytes_v = (unsigned)((bv - av) * sizeof(T));
-    const unsigned bytes_c = (unsigned)((bc - ac) * sizeof(int32_t));
-    mbar_arrive_expect_tx(&bar[w][s], bytes_v + bytes_c);
-    if (bytes_v) bulk_g2s(dv, P.vals + av, bytes_v, &bar[w][s]);
-    if (bytes_c) bulk_g2s(dc, P.cols + ac, bytes_c, &bar[w][s]);
-  };
-
-  if (lane == 0 && P.withhold_ns == 0)
-    for (int s = 0; s < kStgStages; ++s) {
-      const int64_t g = g0 + (int64_t)s * nw;
-      if (g < ngroups) issue(__ldg(&P.ro[g * 32]), __ldg(&P.ro[min(P.n, g * 32 + 32)]), s);
-    }
-  const uint64_t wait_ns = P.withhold_ns ? P.withhold_ns : kWaitLimitNs;
-  double dacc = 0.0;
-  bool ok = true;
-  int it = 0;
-  for (int64_t g = g0; g < ngroups; g += nw, ++it) {
-    const int s = it % kStgStages;
-    const int64_t r = g * 32 + lane;
-    const int64_t gn = g + (int64_t)kStgStages * nw;  // the group stage s takes next
-    // the group's and this lane's row bounds, and lane 0's bounds of the
-    // next group, loaded before the wait so their latency overlaps it (the
-    // next copy then starts as soon as the lanes are done)
-    const int32_t a = __ldg(&P.ro[g * 32]);
-    int32_t ra = 0, rb = 0;
-    if (r < P.n) {
-      ra = __ldg(&P.ro[r]);
-      rb = __ldg(&P.ro[r + 1]);
-    }
-    int64_t na = 0, ne = 0;
-    if (lane == 0 && gn < ngroups) {
-      na = __ldg(&P.ro[gn * 32]);
-      ne = __ldg(&P.ro[min(P.n, gn * 32 + 32)]);
-    }
-    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w][s], (unsigned)((it / kStgStages) & 1), wait_ns));
-    if (!ok) break;
-    if (r < P.n) {
-      const T* rv = reinterpret_cast<const T*>(wbase + (size_t)s * sbytes) + (ra - (a & ~(VA - 1)));
-      const int32_t* rc =
-          reinterpret_cast<const int32_t*>(wbase + (size_t)s * sbytes + vbytes) + (ra - (a & ~3));
-      const T sum = row_dot<T, 27>(rv, rc, rb - ra, P.x);
-      if (MODE == SPMV_RESID) {
-        const double rr = P.b[r] - (double)sum;
-        P.y[r] = (T)rr;
-        dacc = fma(rr, rr, dacc);
-      } else {
-        P.y[r] = sum;
-        if (MODE == SPMV_DOT) dacc = fma((double)sum, (double)__ldg(&P.x[r]), dacc);
-      }
-    }
-    __syncwarp();  // every lane is done reading stage s
-    if (lane == 0 && gn < ngroups) issue(na, ne, s);
-  }
-  if (!ok) {
-    if (lane == 0) {
-      atomicOr(P.err, ERR_WAIT_TIMEOUT);
-      // drain: give each stage with a copy issued a bounded chance to land
-      // before the block exits (an injected fault issued none)
-      for (int j = it; j < it + kStgStages; ++j)
-        if (P.withhold_ns == 0 && g0 + (int64_t)j * nw < ngroups)
-          mbar_wait_bounded(&bar[w][j % kStgStages], (unsigned)((j / kStgStages) & 1));
-    }
-    __syncwarp();
-  }
-  // every warp reaches the block reduction, also after a timeout
-  if (MODE != SPMV_PLAIN) {
-    const double bt = block_sum(dacc, red);
-    double total;
-    if (grid_reduce_last(bt, P.partials, P.ticket, red, &total) && threadIdx.x == 0)
-      spmv_epilogue<MODE>(total, P.cg, P.dot_out);
-  }
+  rank += __popc(same & ((1u << lane) - 1u));
+  lane_of_rank[rank] = (uint8_t)lane;
+  __syncwarp();
+  RowPair q;
+  q.other = lane_of_rank[31 - rank];
+  const int olen = __shfl_sync(0xffffffffu, len, q.other), oen = __shfl_sync(0xffffffffu, en, q.other);
+  const int give = (abs(len - olen)) / 2;
+  q.own = len > olen ? len - give : len;
+  q.extra = len < olen ? give : 0;
+  q.from = oen - give;
+  return q;
 }
 
-// FP64 CSR rows whose longest is not known: staged as in k_spmv_staged, with a
-// stage of `cap` entries (the host's guess from the mean row length).  Groups
-// that do not fit it, or hold a row over twice the unrolled length, read from
-// global memory, a row at a time over the warp.  So no pass over the row
-// offsets and no read-back precede the product: 1.48 M rows of 4 to 27 entries
-// 107 us per call against 121.  What bounds it: row_dot's 27 FMAs per row
-// whatever its length (the FP64 pipe is busy two thirds of the time).  Cutting
-// a group's entries into 32 equal runs instead, a lane per run, took a quarter
-// less of the FP64 pipe but twice the instructions, 147 us.
-constexpr int kAnyLongest = 54;
+// the lane's row times x; gv, gc: the group's staged values and columns
+__device__ __forceinline__ double pair_dot(const RowPair& q, int st, const double* gv, const int32_t* gc,
+                                           const double* __restrict__ x)
+{
+  const int cnt = q.own + q.extra, jump = q.from - st - q.own;
+  double s = 0.0, mine = 0.0;
+#pragma unroll
+  for (int k0 = 0; k0 < kPairSteps; k0 += kPairSteps / 2) {
+    double v[kPairSteps / 2], xv[kPairSteps / 2];
+#pragma unroll
+    for (int k = 0; k < kPairSteps / 2; ++k) {
+      const int i = min(k0 + k, max(cnt - 1, 0)), at = st + i + (i < q.own ? 0 : jump);
+      xv[k] = cnt > 0 ? ld_gather(&x[gc[at]]) : 0.0;
+      v[k] = gv[at];
+    }
+#pragma unroll
+    for (int k = 0; k < kPairSteps / 2; ++k) {
+      if (k0 + k == q.own) {
+        mine = s;
+        s = 0.0;
+      }
+      const double t = fma(v[k], xv[k], s);
+      s = k0 + k < cnt ? t : s;
+    }
+  }
+  if (q.own == kPairSteps) {
+    mine = s;
+    s = 0.0;
+  }
+  const double help = __shfl_sync(0xffffffffu, s, q.other);
+  return mine + help;
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(kStgWarps * 32, 5) k_spmv_any(SpmvParams<double> P, int cap)
+__global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<double> P, int cap)
 {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t bar[kStgWarps][kStgStages];
+  __shared__ uint64_t bar[kStgWarps];
+  __shared__ uint8_t lanes[kStgWarps][32];
   __shared__ double red[32];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   const size_t vbytes = (size_t)cap * sizeof(double);
-  const size_t sbytes = vbytes + (size_t)cap * sizeof(int32_t);
-  unsigned char* wbase = smem + (size_t)w * kStgStages * sbytes;
+  unsigned char* const stage = smem + (size_t)w * (vbytes + (size_t)cap * sizeof(int32_t));
+  double* const dv = reinterpret_cast<double*>(stage);
+  int32_t* const dc = reinterpret_cast<int32_t*>(stage + vbytes);
   const int64_t ngroups = (P.n + 31) / 32;
   const int64_t nw = (int64_t)gridDim.x * kStgWarps;
   const int64_t g0 = (int64_t)blockIdx.x * kStgWarps + w;
   if (lane == 0) {
-    for (int s = 0; s < kStgStages; ++s) mbar_init(&bar[w][s], 1);
+    mbar_init(&bar[w], 1);
     fence_mbar_init();
   }
   __syncthreads();
 
   // up to 3 elements of slack at each end of a group (16-byte boundaries)
   auto staged = [&](int64_t a, int64_t e) { return e - a + 8 <= cap; };
-  // lane 0: nonzeros [a, e) of one group into stage s
-  auto issue = [&](int64_t a, int64_t e, int s) {
+  // lane 0: nonzeros [a, e) of one group into the stage
+  auto issue = [&](int64_t a, int64_t e) {
     if (!staged(a, e)) {
-      mbar_arrive_expect_tx(&bar[w][s], 0);
+      mbar_arrive_expect_tx(&bar[w], 0);
       return;
     }
     const int64_t av = a & ~(int64_t)1, ac = a & ~(int64_t)3;
     const int64_t bv = max(av, min((e + 1) & ~(int64_t)1, P.nnz & ~(int64_t)1));
     const int64_t bc = max(ac, min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3));
-    double* dv = reinterpret_cast<double*>(wbase + (size_t)s * sbytes);
-    int32_t* dc = reinterpret_cast<int32_t*>(wbase + (size_t)s * sbytes + vbytes);
     // ragged tail past the last 16-byte boundary of the arrays: plain loads
     for (int64_t k = bv; k < e; ++k) dv[k - av] = P.vals[k];
     for (int64_t k = bc; k < e; ++k) dc[k - ac] = P.cols[k];
     fence_proxy_async_smem();
     const unsigned bytes_v = (unsigned)((bv - av) * sizeof(double));
     const unsigned bytes_c = (unsigned)((bc - ac) * sizeof(int32_t));
-    mbar_arrive_expect_tx(&bar[w][s], bytes_v + bytes_c);
-    if (bytes_v) bulk_g2s(dv, P.vals + av, bytes_v, &bar[w][s]);
-    if (bytes_c) bulk_g2s(dc, P.cols + ac, bytes_c, &bar[w][s]);
+    mbar_arrive_expect_tx(&bar[w], bytes_v + bytes_c);
+    if (bytes_v) bulk_g2s(dv, P.vals + av, bytes_v, &bar[w]);
+    if (bytes_c) bulk_g2s(dc, P.cols + ac, bytes_c, &bar[w]);
   };
   auto bounds = [&](int64_t g, int64_t& a, int64_t& e) {
     a = __ldg(&P.ro[g * 32]);
     e = __ldg(&P.ro[min(P.n, g * 32 + 32)]);
   };
 
-  if (lane == 0 && P.withhold_ns == 0)
-    for (int s = 0; s < kStgStages; ++s) {
-      const int64_t g = g0 + (int64_t)s * nw;
-      int64_t a, e;
-      if (g < ngroups) {
-        bounds(g, a, e);
-        issue(a, e, s);
-      }
-    }
+  if (lane == 0 && P.withhold_ns == 0 && g0 < ngroups) {
+    int64_t a, e;
+    bounds(g0, a, e);
+    issue(a, e);
+  }
   const uint64_t wait_ns = P.withhold_ns ? P.withhold_ns : kWaitLimitNs;
   double dacc = 0.0;
   bool ok = true;
   int it = 0;
   for (int64_t g = g0; g < ngroups; g += nw, ++it) {
-    const int s = it % kStgStages;
     const int64_t r = g * 32 + lane;
-    const int64_t gn = g + (int64_t)kStgStages * nw;  // the group stage s takes next
+    const int64_t gn = g + nw;  // the group the stage takes next
     int64_t a, e, na = 0, ne = 0;
     bounds(g, a, e);
     const int m = (int)(e - a);
@@ -507,13 +454,15 @@ __global__ void __launch_bounds__(kStgWarps * 32, 5) k_spmv_any(SpmvParams<doubl
       en = (int)(__ldg(&P.ro[r + 1]) - a);
     }
     if (lane == 0 && gn < ngroups) bounds(gn, na, ne);
-    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w][s], (unsigned)((it / kStgStages) & 1), wait_ns));
+    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w], (unsigned)(it & 1), wait_ns));
     if (!ok) break;
     double sum = 0.0;
     if (staged(a, e) && __reduce_max_sync(0xffffffffu, en - st) <= kAnyLongest) {
-      const double* gv = reinterpret_cast<const double*>(wbase + (size_t)s * sbytes) + (a & 1);
-      const int32_t* gc = reinterpret_cast<const int32_t*>(wbase + (size_t)s * sbytes + vbytes) + (a & 3);
-      sum = row_dot<double, 27>(gv + st, gc + st, en - st, P.x);
+      const double* gv = dv + (a & 1);
+      const int32_t* gc = dc + (a & 3);
+      const RowPair q = row_pair(st, en, lanes[w]);
+      if (__reduce_max_sync(0xffffffffu, q.own + q.extra) <= kPairSteps) sum = pair_dot(q, st, gv, gc, P.x);
+      else sum = row_dot<double, 27>(gv + st, gc + st, en - st, P.x);
     } else {
       for (int j = 0; j < 32; ++j) {
         const int js = __shfl_sync(0xffffffffu, st, j), je = __shfl_sync(0xffffffffu, en, j);
@@ -533,17 +482,15 @@ __global__ void __launch_bounds__(kStgWarps * 32, 5) k_spmv_any(SpmvParams<doubl
         if (MODE == SPMV_DOT) dacc = fma(sum, __ldg(&P.x[r]), dacc);
       }
     }
-    __syncwarp();  // every lane is done reading stage s
-    if (lane == 0 && gn < ngroups) issue(na, ne, s);
+    __syncwarp();  // every lane is done reading the stage
+    if (lane == 0 && gn < ngroups) issue(na, ne);
   }
   if (!ok) {
     if (lane == 0) {
       atomicOr(P.err, ERR_WAIT_TIMEOUT);
-      // drain: give each stage with a copy issued a bounded chance to land
-      // before the block exits (an injected fault issued none)
-      for (int j = it; j < it + kStgStages; ++j)
-        if (P.withhold_ns == 0 && g0 + (int64_t)j * nw < ngroups)
-          mbar_wait_bounded(&bar[w][j % kStgStages], (unsigned)((j / kStgStages) & 1));
+      // drain: give the copy a bounded chance to land before the block exits (an
+      // injected fault issued none)
+      if (P.withhold_ns == 0) mbar_wait_bounded(&bar[w], (unsigned)(it & 1));
     }
     __syncwarp();
   }
@@ -817,15 +764,15 @@ mfe_status take_wait_injection(mfe_ctx* ctx, uint64_t* withhold_ns)
 }
 
 template <typename T>
-static size_t staged_smem(int max_len, bool ell)
+static size_t staged_smem(int K)
 {
-  return (size_t)kStgWarps * kStgStages * stg_cap(max_len, ell) * (sizeof(T) + sizeof(int32_t));
+  return (size_t)kStgWarps * kStgStages * stg_cap(K, true) * (sizeof(T) + sizeof(int32_t));
 }
 
 template <typename T>
-static int staged_grid(mfe_ctx* ctx, int64_t nrows, int max_len, bool ell)
+static int staged_grid(mfe_ctx* ctx, int64_t nrows, int K)
 {
-  const size_t smem = staged_smem<T>(max_len, ell);
+  const size_t smem = staged_smem<T>(K);
   const int per_sm = std::max(1, std::min(16, (int)((227 * 1024) / (smem + 1024))));
   return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)kStgWarps),
                                                      (int64_t)ctx->sm_count * per_sm));
@@ -842,41 +789,31 @@ static mfe_status staged_configure(mfe_ctx* ctx, const void* kernel, size_t smem
   return MFE_OK;
 }
 
-// P filled but for cap; rows of at most max_len <= kStgMaxLen entries
-template <typename T, int MODE>
-static mfe_status launch_staged(mfe_ctx* ctx, SpmvParams<T>& P, int max_len)
+// k_spmv_any for n rows with nnz entries, at most max_len each (<= 0: not known):
+// the stage holds 1.25 times the mean and two entries more per row, 32 at most
+// (rows of independent lengths hardly ever fill it: 720 of 752 entries at most
+// over 46,000 groups of rows of 4 to 27)
+static int any_cap(int64_t n, int64_t nnz, int max_len)
 {
-  static bool configured[64] = {};
-  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_staged<T, MODE>,
-                           staged_smem<T>(kStgMaxLen, false), configured));
-  P.cap = stg_cap(max_len, false);
-  MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
-  k_spmv_staged<T, MODE><<<staged_grid<T>(ctx, P.n, max_len, false), kStgWarps * 32,
-                           staged_smem<T>(max_len, false), ctx->stream>>>(P, max_len);
-  return check_launch(ctx, "k_spmv_staged");
+  const int most = max_len > 0 ? std::min(max_len, kStgMaxLen) : kStgMaxLen;
+  return stg_cap(std::max(1, std::min(most, (int)(1.25 * (double)nnz / (double)std::max<int64_t>(n, 1)) + 2)), false);
 }
 
-// k_spmv_any for rows of mean length `mean`: the stage holds 1.3 times the
-// mean and two entries more per row, 32 at most (rows of independent lengths
-// hardly ever fill it: 720 of 800 entries at most over 46,000 groups of rows of
-// 4 to 27)
-static int any_cap(double mean) { return stg_cap(std::max(1, std::min(kStgMaxLen, (int)(1.3 * mean) + 2)), false); }
-
-static size_t any_smem(int cap) { return (size_t)kStgWarps * kStgStages * cap * (sizeof(double) + sizeof(int32_t)); }
+static size_t any_smem(int cap) { return (size_t)kStgWarps * cap * (sizeof(double) + sizeof(int32_t)); }
 
 static int any_grid(mfe_ctx* ctx, int64_t nrows, int cap)
 {
-  const int per_sm = std::max(1, std::min(16, (int)((227 * 1024) / (any_smem(cap) + 3072))));
+  const int per_sm = std::max(1, std::min(kAnyBlocks, (int)((228 * 1024) / (any_smem(cap) + 1024 + 512))));
   return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)kStgWarps),
                                                      (int64_t)ctx->sm_count * per_sm));
 }
 
 template <int MODE>
-static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<double>& P)
+static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<double>& P, int max_len)
 {
   static bool configured[64] = {};
   MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<MODE>, any_smem(stg_cap(kStgMaxLen, false)), configured));
-  const int cap = any_cap((double)P.nnz / (double)P.n);
+  const int cap = any_cap(P.n, P.nnz, max_len);
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
   k_spmv_any<MODE><<<any_grid(ctx, P.n, cap), kStgWarps * 32, any_smem(cap), ctx->stream>>>(P, cap);
   return check_launch(ctx, "k_spmv_any");
@@ -889,9 +826,7 @@ int spmv_grid(mfe_ctx* ctx, const mfe_csr* A)
     return (int)std::max<int64_t>(
         1, std::min<int64_t>(ceil_div(A->nrows * 32, 256), (int64_t)ctx->sm_count * 8));
   if (A->dtype == MFE_F64) {
-    if (A->max_row_len <= 0)
-      return any_grid(ctx, A->nrows, any_cap((double)A->nnz / std::max<int64_t>(A->nrows, 1)));
-    return staged_grid<double>(ctx, A->nrows, max_len, false);
+    return any_grid(ctx, A->nrows, any_cap(A->nrows, A->nnz, A->max_row_len));
   }
   const int rows = tile_rows();
   const int64_t ntiles = ceil_div(A->nrows, rows);
@@ -945,8 +880,7 @@ static mfe_status launch_t(mfe_ctx* ctx, const mfe_csr* A, const T* x, T* y, con
   if (A->nrows == 0) return MFE_OK;
   if (max_len <= kStgMaxLen && aligned16(A->vals) && aligned16(A->cols)) {
     if constexpr (sizeof(T) == 8) {
-      if (max_len <= 0) return launch_any<MODE>(ctx, P);
-      return launch_staged<T, MODE>(ctx, P, max_len);
+      return launch_any<MODE>(ctx, P, max_len);
     } else {
       MFE_CUDA_TRY(ctx, configure_tiled(ctx->device));
       const size_t smem = tiled_smem<T>(rows, std::max(max_len, 1));
@@ -1006,7 +940,7 @@ static mfe_status launch_ell_t(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y,
                                const double* b, CgState* cg)
 {
   static bool configured[64] = {};
-  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_ell<T, MODE>, staged_smem<T>(kStgMaxLen, true),
+  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_ell<T, MODE>, staged_smem<T>(kStgMaxLen),
                            configured));
   SpmvParams<T> P;
   memset(&P, 0, sizeof(P));
@@ -1027,7 +961,7 @@ static mfe_status launch_ell_t(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y,
   if (cg) P.err = &cg->err;
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
   const int K = E->ncols_per_row;
-  k_spmv_ell<T, MODE><<<staged_grid<T>(ctx, P.n, K, true), kStgWarps * 32, staged_smem<T>(K, true),
+  k_spmv_ell<T, MODE><<<staged_grid<T>(ctx, P.n, K), kStgWarps * 32, staged_smem<T>(K),
                         ctx->stream>>>(P, K);
   return check_launch(ctx, "k_spmv_ell");
 }

@@ -1,6 +1,6 @@
-"""FP64 products with CSR rows of unknown lengths (k_spmv_any): empty rows, groups
-of 32 rows larger than the stage, long rows among short ones, the last partial
-group, and the dot's epilogue.
+"""FP64 products with CSR rows of any lengths (k_spmv_any): rows in pairs and alone,
+empty rows, groups of 32 rows larger than the stage, long rows among short ones,
+the last partial group, and the dot's epilogue.
 
 Bound: each row is at most its length in FMAs plus the additions that join its
 partial sums (32 at most), every rounding at most 2^-53 of the sum of |a||x| so far:
@@ -19,6 +19,10 @@ import minife_gb300 as M  # noqa: E402
 
 SHAPES = {
     "ragged": lambda r, n: r.integers(4, 28, n),
+    # pairs of rows: 18 entries a lane, 19 (no pairs), the longest that pairs take
+    "0 and 36": lambda r, n: np.arange(n) % 2 * 36,
+    "0 and 37": lambda r, n: np.arange(n) % 2 * 37,
+    "one of 54 in 4": lambda r, n: np.where(np.arange(n) % 4 == 1, 54, 2),
     "even": lambda r, n: np.full(n, 27),
     "short": lambda r, n: r.integers(0, 3, n),
     "one long row per group": lambda r, n: np.where(np.arange(n) % 32 == 17, 200, 1),
