@@ -285,7 +285,6 @@ __global__ void __launch_bounds__(ROWS, 2) k_spmv_tiled(SpmvParams<T> P)
 // behind block barriers (FP32 rows, half the bytes per stage, stay on the tiled
 // kernel).
 constexpr int kStgWarps = 2;    // warps per block
-constexpr int kStgStages = 2;   // stages per warp
 constexpr int kStgMaxLen = 32;  // longer rows: the warp-per-row kernel
 
 // Stage capacity (elements) for a group of 32 rows of at most max_len
@@ -519,23 +518,30 @@ constexpr int ell_min_blocks()
   return sizeof(T) == 4 ? 5 : 0;
 }
 
-template <typename T, int MODE>
+// NS: stages per warp.  FP64 rows in numbers take one, which lets twice as many
+// warps share an SM (ten blocks of two at K = 27): 1.48 M rows 99.7 / 93.8 us,
+// 3.44 M 215 / 189, 8.12 M 515 / 428; 0.75 M 54.3 / 54.2, 0.53 M 41.7 / 43.4.
+// FP32 rows two (1.48 M 52.3 / 62.9).  (One stage and seven to ten blocks per SM
+// in the launch bounds, 64 registers for 56: 1.48 M 99.6-102.8.)
+constexpr int64_t kEllOneStage = 1000000;
+
+template <typename T, int MODE, int NS>
 __global__ void __launch_bounds__(kStgWarps * 32, ell_min_blocks<T>()) k_spmv_ell(SpmvParams<T> P, int K)
 {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t bar[kStgWarps][kStgStages];
+  __shared__ uint64_t bar[kStgWarps][NS];
   __shared__ double red[32];
   constexpr int VA = 16 / sizeof(T);
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   const size_t sbytes = (size_t)32 * K * (sizeof(T) + sizeof(int32_t));
   const size_t vbytes = (size_t)32 * K * sizeof(T);
-  unsigned char* wbase = smem + (size_t)w * kStgStages * sbytes;
+  unsigned char* wbase = smem + (size_t)w * NS * sbytes;
   const int64_t ngroups = (P.n + 31) / 32;
   const int64_t nw = (int64_t)gridDim.x * kStgWarps;
   const int64_t g0 = (int64_t)blockIdx.x * kStgWarps + w;
   if (lane == 0) {
-    for (int s = 0; s < kStgStages; ++s) mbar_init(&bar[w][s], 1);
+    for (int s = 0; s < NS; ++s) mbar_init(&bar[w][s], 1);
     fence_mbar_init();
   }
   __syncthreads();
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(kStgWarps * 32, ell_min_blocks<T>()) k_spmv_el
     if (bytes_c) bulk_g2s(dc, P.cols + a, bytes_c, &bar[w][s]);
   };
   if (lane == 0 && P.withhold_ns == 0)
-    for (int s = 0; s < kStgStages; ++s) {
+    for (int s = 0; s < NS; ++s) {
       const int64_t g = g0 + (int64_t)s * nw;
       if (g < ngroups) issue(g, s);
     }
@@ -568,8 +574,8 @@ __global__ void __launch_bounds__(kStgWarps * 32, ell_min_blocks<T>()) k_spmv_el
   bool ok = true;
   int it = 0;
   for (int64_t g = g0; g < ngroups; g += nw, ++it) {
-    const int s = it % kStgStages;
-    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w][s], (unsigned)((it / kStgStages) & 1), wait_ns));
+    const int s = it % NS;
+    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w][s], (unsigned)((it / NS) & 1), wait_ns));
     if (!ok) break;
     const int64_t r = g * 32 + lane;
     if (r < P.n) {
@@ -586,15 +592,15 @@ __global__ void __launch_bounds__(kStgWarps * 32, ell_min_blocks<T>()) k_spmv_el
       }
     }
     __syncwarp();  // every lane is done reading stage s
-    const int64_t gn = g + (int64_t)kStgStages * nw;
+    const int64_t gn = g + (int64_t)NS * nw;
     if (lane == 0 && gn < ngroups) issue(gn, s);
   }
   if (!ok) {
     if (lane == 0) {
       atomicOr(P.err, ERR_WAIT_TIMEOUT);
-      for (int j = it; j < it + kStgStages; ++j)
+      for (int j = it; j < it + NS; ++j)
         if (P.withhold_ns == 0 && g0 + (int64_t)j * nw < ngroups)
-          mbar_wait_bounded(&bar[w][j % kStgStages], (unsigned)((j / kStgStages) & 1));
+          mbar_wait_bounded(&bar[w][j % NS], (unsigned)((j / NS) & 1));
     }
     __syncwarp();
   }
@@ -763,16 +769,16 @@ mfe_status take_wait_injection(mfe_ctx* ctx, uint64_t* withhold_ns)
   return MFE_OK;
 }
 
-template <typename T>
-static size_t staged_smem(int K)
+template <typename T, int NS>
+static size_t ell_smem(int K)
 {
-  return (size_t)kStgWarps * kStgStages * stg_cap(K, true) * (sizeof(T) + sizeof(int32_t));
+  return (size_t)kStgWarps * NS * stg_cap(K, true) * (sizeof(T) + sizeof(int32_t));
 }
 
-template <typename T>
-static int staged_grid(mfe_ctx* ctx, int64_t nrows, int K)
+template <typename T, int NS>
+static int ell_grid(mfe_ctx* ctx, int64_t nrows, int K)
 {
-  const size_t smem = staged_smem<T>(K);
+  const size_t smem = ell_smem<T, NS>(K);
   const int per_sm = std::max(1, std::min(16, (int)((227 * 1024) / (smem + 1024))));
   return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)kStgWarps),
                                                      (int64_t)ctx->sm_count * per_sm));
@@ -935,12 +941,12 @@ mfe_status launch_spmv(mfe_ctx* ctx, const mfe_csr* A, const void* x, void* y,
   return fail(ctx, MFE_BAD_ARG, "unknown matrix dtype");
 }
 
-template <typename T, int MODE>
-static mfe_status launch_ell_t(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y, const DotSink* sink,
-                               const double* b, CgState* cg)
+template <typename T, int MODE, int NS>
+static mfe_status launch_ell_ns(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y, const DotSink* sink,
+                                const double* b, CgState* cg)
 {
   static bool configured[64] = {};
-  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_ell<T, MODE>, staged_smem<T>(kStgMaxLen),
+  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_ell<T, MODE, NS>, ell_smem<T, NS>(kStgMaxLen),
                            configured));
   SpmvParams<T> P;
   memset(&P, 0, sizeof(P));
@@ -961,9 +967,17 @@ static mfe_status launch_ell_t(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y,
   if (cg) P.err = &cg->err;
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
   const int K = E->ncols_per_row;
-  k_spmv_ell<T, MODE><<<staged_grid<T>(ctx, P.n, K), kStgWarps * 32, staged_smem<T>(K),
+  k_spmv_ell<T, MODE, NS><<<ell_grid<T, NS>(ctx, P.n, K), kStgWarps * 32, ell_smem<T, NS>(K),
                         ctx->stream>>>(P, K);
   return check_launch(ctx, "k_spmv_ell");
+}
+
+template <typename T, int MODE>
+static mfe_status launch_ell_t(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y, const DotSink* sink,
+                               const double* b, CgState* cg)
+{
+  if (sizeof(T) == 8 && E->nrows >= kEllOneStage) return launch_ell_ns<T, MODE, 1>(ctx, E, x, y, sink, b, cg);
+  return launch_ell_ns<T, MODE, 2>(ctx, E, x, y, sink, b, cg);
 }
 
 mfe_status launch_spmv_ell(mfe_ctx* ctx, const mfe_ell* E, const void* x, void* y,
