@@ -638,7 +638,7 @@ def bench_next_rows(args, world, stream, A, b):
                            "spmv": {"ms": t_gmv * 1e3, "bytes": gen_bytes,
                                     "achieved_gbs": gen_bytes / t_gmv / 1e9, "peak_gbs": peak,
                                     "frac": gen_bytes / t_gmv / 1e9 / peak,
-                                    "kernel": "k_spmv_staged (a warp per 32-row group)"}},
+                                    "kernel": "k_spmv_any (a warp per 32-row group, rows in pairs)"}},
     }
 
 

@@ -355,7 +355,8 @@ typedef enum mfe_inner_operator {
  * (x0 copied to p, r = b - A p, then per iteration p update, A p, p.Ap,
  * breakdown test, x and r updates), with matvec_std on the CSR values or,
  * for verified miniFE box operators, the FP64 stencil operator
- * (opts->f64_operator); the loop runs on the device inside one CUDA graph (a
+ * (opts->f64_operator); the loop runs on the device, in one cooperative
+ * kernel (box matrices with short iterations) or inside one CUDA graph (a
  * conditional while node), with no host round trip per iteration. */
 mfe_status mfe_cg_solve(mfe_ctx* ctx, const mfe_csr* A, const double* b, double* x,
                         const mfe_cg_opts* opts, mfe_cg_result* result);

@@ -537,7 +537,7 @@ mfe_status mfe_spmv_stencil64(mfe_ctx* ctx, const mfe_stencil64* S, const double
   A.box_ny = S->box_ny;
   A.box_nz = S->box_nz;
   A.dtype = MFE_F64;
-  return launch_spmv_st64(ctx, &A, S->w, S->dd, x, y, nullptr, nullptr);
+  return launch_spmv_st64(ctx, &A, S->w, S->dd, x, y, nullptr);
 }
 
 mfe_status mfe_gather(mfe_ctx* ctx, int64_t n, const int32_t* idx, const double* x, double* out)

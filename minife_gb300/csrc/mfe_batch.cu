@@ -2,8 +2,9 @@
 // nx x ny x nz box, k = 1, the reference's boundary conditions) assembled
 // into one concatenated store and solved with CG, all boxes advancing
 // together: every iteration is one fixed sequence of launches over all
-// boxes that are still iterating, captured once as a CUDA graph with a
-// conditional while node.
+// boxes that are still iterating, captured as a CUDA graph with a conditional
+// while node whose body holds several iterations (those after the last return
+// at once).
 //
 // HBM layout.  Box b owns rows [row_base_b, row_base_b + n_b) of every
 // concatenated vector and values [nnz_base_b, nnz_base_b + nnz_b) of the

@@ -5,7 +5,9 @@
 // iteration.  Here one iteration is three kernels with the reductions fused
 // into the producers of their operands:
 //   k_cg_p       p = r + beta p                  (p = r at k = 1)
-//   k_spmv_tiled Ap = A p, p.Ap                  (mfe_spmv.cu, SPMV_DOT)
+//   the product  Ap = A p, p.Ap                  (k_spmv_fixed, mfe_fixed64.cu, on a
+//                verified stencil; k_spmv_box, mfe_spmv_box.cu, with a box's
+//                values; k_spmv_sell, mfe_ell.cu, or mfe_spmv.cu otherwise)
 //   k_cg_update  x += alpha p, r -= alpha Ap, r.r, scalar bookkeeping
 // i.e. 11 vector passes per iteration plus one read of the matrix.  The loop
 // itself is a CUDA graph with a conditional while node: the last block of
@@ -14,6 +16,9 @@
 // one graph launch with no host round trip.  The breakdown test
 // (cg_solve.hpp:186-198) needs two extra norms; when its pre-test fires the
 // graph exits and the host finishes that iteration with separate kernels.
+//
+// Box matrices whose iterations are short run them in one cooperative kernel
+// instead of the graph (mfe_cg_loop.cu).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>

@@ -195,10 +195,9 @@ bool stencil64_host_classes(int Nx, int Ny, int Nz, const double* vals, double* 
 mfe_status stencil64_verify_on(mfe_ctx* ctx, cudaStream_t s, int Nx, int Ny, int Nz,
                                const double* vals, const double* table, unsigned* bad);
 // y = S x in FP64 on natural-layout vectors (A's box dimensions), with x.y
-// into the CG state (pAp and the breakdown pre-test) when cg_state is set,
-// else into sink->out (when sink is set)
+// into sink->out when sink is set
 mfe_status launch_spmv_st64(mfe_ctx* ctx, const mfe_csr* A, const double* w8, double dd,
-                            const double* x, double* y, const DotSink* sink, void* cg_state);
+                            const double* x, double* y, const DotSink* sink);
 
 // ---- the FP64 CG's product in fixed point (mfe_fixed64.cu) ----
 // Ap = S p with the same operator on the integer pipe, p.Ap and the breakdown

@@ -227,7 +227,7 @@ mfe_status cg_jacobi(mfe_ctx* ctx, const mfe_csr* A, const double* b, double* x,
 
   auto body = [&](cudaGraphConditionalHandle h, int in_graph) -> mfe_status {
     if (st64)
-      MFE_TRY(launch_spmv_st64(ctx, A, w8, dd, p, Ap, &ps, nullptr));
+      MFE_TRY(launch_spmv_st64(ctx, A, w8, dd, p, Ap, &ps));
     else
       MFE_TRY(launch_spmv(ctx, A, p, Ap, &ps, nullptr, nullptr));
     k_pcg_update<<<vg, kPT, 0, ctx->stream>>>(n, x, r, z, p, Ap, dinv, st, partials, tickets, h,

@@ -13,8 +13,8 @@
 // (|dz|, |dy|, |dx|) only.  stencil64_prepare (mfe_stencil.cu) checks this
 // on the matrix itself on every solve, every entry within 2^-40 of its row's
 // largest magnitude (the assembled entries of one class differ by rounding
-// only: up to a few hundred ulps, 1e-13 relative), and the CG then applies
-// the operator from its eight class weights w[4|dz| + 2|dy| + |dx|] and dd.
+// only: up to a few hundred ulps, 1e-13 relative); the operator then is its
+// eight class weights w[4|dz| + 2|dy| + |dx|] and dd.
 //
 // A row as separable sums (x~ = x with the Dirichlet nodes zeroed):
 //   per plane z and position p: a = x~[p], sx = x~[p-1] + x~[p+1],
@@ -28,7 +28,7 @@
 // P1 and 16 FMAs for Q, and a row 1 final addition and 1 FMA for p.Ap: 13.5
 // FP64 operations per row instead of the CSR kernel's 28.
 //
-// k_spmv_st64 works on the CG's natural-layout vectors.  A CTA owns 1024
+// k_spmv_st64 works on natural-layout vectors.  A CTA owns 1024
 // consecutive positions of the xy plane (four per thread) and a run of z
 // steps; the (plane tile, z) steps are split evenly over the grid.  Each
 // thread reads its 3 x 6 window x[p-1 .. p+4] of lines y-1, y, y+1 of each
@@ -45,7 +45,6 @@
 #include <cmath>
 #include <type_traits>
 
-#include "mfe_cgstate.cuh"
 #include "mfe_common.cuh"
 #include "mfe_internal.h"
 
@@ -64,7 +63,6 @@ struct St64Params {
   double* partials;
   unsigned* ticket;
   double* dot_out;
-  CgState* cg;
 };
 
 // CTAs per SM of the grid (three fit at the 76 registers ptxas picks with no
@@ -249,14 +247,7 @@ __global__ void __launch_bounds__(kT64, kSt64CtasPerSm) k_spmv_st64(const __grid
   if (!DOT) return;
   const double bt = block_sum(dacc, red);
   double total;
-  if (grid_reduce_last(bt, P.partials, P.ticket, red, &total) && threadIdx.x == 0) {
-    if (P.cg != nullptr) {
-      P.cg->pAp = total;
-      if (total < P.cg->brkdown_tol) P.cg->check_pending = 1;
-    } else {
-      *P.dot_out = total;
-    }
-  }
+  if (grid_reduce_last(bt, P.partials, P.ticket, red, &total) && threadIdx.x == 0) *P.dot_out = total;
 }
 
 // four positions per thread: measured at 256^3, 0.484 ms per product
@@ -280,7 +271,7 @@ mfe_status st64_launch(mfe_ctx* ctx, St64Params& P)
 }  // namespace
 
 mfe_status launch_spmv_st64(mfe_ctx* ctx, const mfe_csr* A, const double* w8, double dd,
-                            const double* x, double* y, const DotSink* sink, void* cg_state)
+                            const double* x, double* y, const DotSink* sink)
 {
   St64Params P;
   P.Nx = A->box_nx + 1;
@@ -291,11 +282,10 @@ mfe_status launch_spmv_st64(mfe_ctx* ctx, const mfe_csr* A, const double* w8, do
   P.dd = dd;
   P.x = x;
   P.y = y;
-  P.cg = static_cast<CgState*>(cg_state);
   P.partials = sink ? sink->partials : nullptr;
   P.ticket = sink ? sink->ticket : nullptr;
-  P.dot_out = sink && !cg_state ? sink->out : nullptr;
-  const bool dot = P.cg || P.dot_out;
+  P.dot_out = sink ? sink->out : nullptr;
+  const bool dot = P.dot_out != nullptr;
   if (dot && (!P.partials || !P.ticket))
     return fail(ctx, MFE_BAD_ARG, "stencil SpMV: a dot needs reduction buffers");
   return dot ? st64_launch<true>(ctx, P) : st64_launch<false>(ctx, P);
