@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 
 #include "mfe_common.cuh"
 #include "mfe_internal.h"
@@ -103,6 +104,19 @@ inline size_t plan_held(int64_t n, int g, size_t elem, size_t room, int most, in
   return elem * *span * *held;
 }
 
+// A loop's blocks fill the device and wait for one another, so two of them must
+// never hold parts of it: each launch, of any context and stream, waits on the
+// device for the one before it.
+struct LoopOrder {
+  std::mutex mu;
+  cudaEvent_t last = nullptr;
+};
+inline LoopOrder& loop_order(int device)
+{
+  static LoopOrder order[64];
+  return order[device & 63];
+}
+
 // The attribute set and the occupancy asked for, once per kernel and device; a
 // launch of blocks that would not all be resident is refused.
 template <size_t kMost>
@@ -117,7 +131,12 @@ inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads
     if (blocks < per_sm) return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
     have.store(blocks, std::memory_order_release);
   }
+  LoopOrder& order = loop_order(ctx->device);
+  std::lock_guard<std::mutex> lock(order.mu);
+  if (!order.last) MFE_CUDA_TRY(ctx, cudaEventCreateWithFlags(&order.last, cudaEventDisableTiming));
+  MFE_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, order.last, 0));
   MFE_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream));
+  MFE_CUDA_TRY(ctx, cudaEventRecord(order.last, ctx->stream));
   return MFE_OK;
 }
 
