@@ -42,7 +42,7 @@
 // range are formed in FP64 (row_fp64).
 //
 // A CTA owns up to 4 NT consecutive positions of the xy plane and marches
-// along z; the (plane tile, z) steps are split evenly over the grid.  Per
+// along z; the (plane tile, z) steps are shared out over the grid (fx_setup).  Per
 // plane, with one barrier: the next plane's window (the tile and one line and
 // one position on either side) is loaded coalesced while the current one is
 // computed, then split into the other half of a two-plane buffer, and the
@@ -54,17 +54,19 @@
 // then per block and over the grid in block order (deterministic for a fixed
 // grid).
 //
-// Measured at 256^3 in the solve: 0.234 ms against 0.508 ms; the solve of an
-// N(0, 1) right-hand side to 2e-11 takes 0.42 ms per iteration instead of
-// 0.70.  What bounds it: the integer pipe.  A row costs about 190 instructions;
-// IMAD.WIDE and the ALU's instructions share one rate of 64 per clock and SM
-// (microbenchmark: alternating LOP3 and IMAD.WIDE issue 2.0 per clock and SM
-// together, as either alone), of which 62 % are used, the rest lost to the
-// per-plane barrier and shared-memory queueing at 16 warps per SM.  Tried and
-// slower: exponents per row instead of per thread (0.34 ms without the dot
-// against 0.19), the p and x updates fused into the staging pass (0.36 ms and
-// more: its FP64 work then queues before the integer work of the same warps),
-// and the same with dedicated staging warps (0.37 ms).
+// Measured at 256^3 in the solve: 0.218 ms against 0.508 ms; the solve of an
+// N(0, 1) right-hand side to 2e-11 takes 0.40 ms per iteration instead of
+// 0.70.  What bounds it: the integer pipe and, at 16 warps per SM, latency.  A row
+// costs about 200 instructions; IMAD.WIDE and the ALU's instructions share one
+// rate of 64 per clock and SM (microbenchmark: alternating LOP3 and IMAD.WIDE
+// issue 2.0 per clock and SM together, as either alone).  At 200^3 the ALU pipe
+// is busy 47 % of the time, the FP64 pipe (conversions, p.Ap) 44 %, the rest goes to the
+// per-plane barrier and shared-memory queueing.  Tried and slower: exponents per
+// row instead of per thread (0.34 ms without the dot against 0.19), the p and x
+// updates fused into the staging pass (0.36 ms and more: its FP64 work then
+// queues before the integer work of the same warps), the same with dedicated
+// staging warps (0.37 ms), and x += alpha p of the iteration before carried by
+// the rows written out (0.30 ms, of which the update kernel gives back 0.04).
 #pragma once
 
 #include <algorithm>
