@@ -25,6 +25,7 @@
 // deterministically (fixed grid, last block sums the block partials in order).
 // Matrices with rows longer than 32 entries use a warp-per-row kernel.
 #include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -302,7 +303,8 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // mean row length): twenty-four warps per SM, a part of them computing while the
 // others' next groups arrive.  Groups that do not fit the stage, or hold a row
 // over kAnyLongest, read from global memory, a row at a time over the warp, so
-// the longest row need not be known.
+// the longest row need not be known.  `most`: what a group may take up when it is
+// (INT_MAX else); more is an error in the caller's max_row_len, and recorded.
 //
 // What bounds it: the FP64 pipe, whose instructions take 17 clocks an SM whatever
 // the number of lanes at work.  Hence the rows in pairs (row_pair): 1.48 M rows
@@ -385,7 +387,7 @@ __device__ __forceinline__ double pair_dot(const RowPair& q, int st, const doubl
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<double> P, int cap)
+__global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<double> P, int cap, int most)
 {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t bar[kStgWarps];
@@ -410,13 +412,14 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
   auto staged = [&](int64_t a, int64_t e) { return e - a + 8 <= cap; };
   // lane 0: nonzeros [a, e) of one group into the stage
   auto issue = [&](int64_t a, int64_t e) {
+    const int64_t av = a & ~(int64_t)1, ac = a & ~(int64_t)3;
+    const int64_t bv = max(av, min((e + 1) & ~(int64_t)1, P.nnz & ~(int64_t)1));
+    const int64_t bc = max(ac, min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3));
+    if (max(bv, e) - av > most || max(bc, e) - ac > most) atomicOr(P.err, ERR_TILE_OVERFLOW);
     if (!staged(a, e)) {
       mbar_arrive_expect_tx(&bar[w], 0);
       return;
     }
-    const int64_t av = a & ~(int64_t)1, ac = a & ~(int64_t)3;
-    const int64_t bv = max(av, min((e + 1) & ~(int64_t)1, P.nnz & ~(int64_t)1));
-    const int64_t bc = max(ac, min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3));
     // ragged tail past the last 16-byte boundary of the arrays: plain loads
     for (int64_t k = bv; k < e; ++k) dv[k - av] = P.vals[k];
     for (int64_t k = bc; k < e; ++k) dc[k - ac] = P.cols[k];
@@ -821,7 +824,8 @@ static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<double>& P, int max_len)
   MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<MODE>, any_smem(stg_cap(kStgMaxLen, false)), configured));
   const int cap = any_cap(P.n, P.nnz, max_len);
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
-  k_spmv_any<MODE><<<any_grid(ctx, P.n, cap), kStgWarps * 32, any_smem(cap), ctx->stream>>>(P, cap);
+  k_spmv_any<MODE><<<any_grid(ctx, P.n, cap), kStgWarps * 32, any_smem(cap), ctx->stream>>>(
+      P, cap, max_len > 0 ? stg_cap(max_len, false) : INT_MAX);
   return check_launch(ctx, "k_spmv_any");
 }
 

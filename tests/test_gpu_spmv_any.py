@@ -58,3 +58,29 @@ def test_uneven_rows(shape, n):
         d = M.matvec_and_dot(A, dev[3], y)
         yy = y.cpu().numpy()
         assert abs(d - float(np.dot(yy.astype(np.longdouble), x))) <= (n + 64) * 2.0**-53 * float(np.abs(yy * x).sum())
+
+
+@pytest.mark.parametrize("stated,refused", [(27, False), (26, False), (25, True), (4, True)])
+def test_stated_longest_row(stated, refused):
+    # one row of 27 per group of 32, the others of 25 (26 where 25 is stated): 802
+    # or 833 entries a group, where 32 rows of the stated length may take 872, 840,
+    # 808 and 136 with the rounding to 16 bytes
+    n = 32 * 50
+    lens = np.where(np.arange(n) % 32 == 3, 27, 26 if refused and stated == 25 else 25)
+    ro = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    rng = np.random.default_rng(5)
+    cols, vals, x = rng.integers(0, n, ro[-1]).astype(np.int32), rng.normal(size=ro[-1]), rng.normal(size=n)
+    dev = [torch.from_numpy(a).cuda() for a in (ro, cols, vals, x)]
+    A = M.CSRMatrix(*dev[:3], max_row_len=stated)
+    ctx = M.Context()
+    y = torch.empty_like(dev[3])
+    M.matvec(A, dev[3], y, ctx=ctx)
+    if refused:
+        with pytest.raises(M.MiniFEError):
+            ctx.synchronize()
+    else:
+        ctx.synchronize()
+        ref = np.add.reduceat(vals * x[cols], ro[:-1])
+        size = np.add.reduceat(np.abs(vals * x[cols]), ro[:-1])
+        assert (np.abs(y.cpu().numpy() - ref) <= 2 * (27 + 32) * 2.0**-53 * size).all()
+    ctx.close()
