@@ -163,6 +163,15 @@ mfe_status mfe_ctx_create(int device, mfe_ctx** out)
     return MFE_CUDA_ERR;
   }
   ctx->stream = ctx->own_stream;
+  // the products' error word starts at zero (memory may come with what another
+  // context left in it)
+  void* err = workspace(ctx, "spmv.err", sizeof(unsigned));
+  if (!err || cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
+      cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    cudaGetLastError();
+    mfe_ctx_destroy(ctx);
+    return MFE_CUDA_ERR;
+  }
   *out = ctx;
   return MFE_OK;
 }
