@@ -2,28 +2,19 @@
 //
 // GB300 has a reduced FP64 pipe (about 2 FP64 FMA per clock per SM), which
 // puts an FP64 CSR SpMV close to the FP64 issue limit as well as the HBM
-// limit.  The main kernel therefore spends exactly one FP64 FMA per nonzero:
-// one thread owns one row and accumulates it sequentially (no shuffle-add
-// trees, which would cost 5 extra FP64 adds per lane), while the row's values
-// and column indices arrive through shared memory so the HBM reads stay fully
-// coalesced:
-//   - a persistent grid walks tiles of ROWS consecutive rows; the nonzeros of
-//     a tile are contiguous in CSR, so one thread issues two 1-D bulk async
-//     copies (TMA, cp.async.bulk) for the tile's values and columns into a
-//     shared-memory stage, completion tracked by an mbarrier;
-//   - S stages are in flight per CTA, so the copies for the next tiles
-//     overlap the current tile's FMAs;
-//   - x is gathered through the read-only path (27-point rows touch three
-//     x-planes, which stay L1/L2 resident).
-// Two forms of that scheme: FP64 rows go through the warp-staged kernel (a
-// warp per 32-row group with its own ring of stages and mbarriers, no block
-// barrier), FP32 rows through the tiled kernel (a block per 128-row tile).
-// The reference's row-major ELLMatrix has its own warp-staged kernel, whose
-// groups start aligned.
+// limit.  The main kernel (k_spmv_any) therefore sums a row in one lane or two
+// (no shuffle-add trees, which would cost 5 extra FP64 adds per lane), while the
+// values and column indices of 32 rows arrive in a warp's own shared memory by
+// two 1-D bulk async copies (TMA, cp.async.bulk) tracked by an mbarrier, so the
+// HBM reads stay fully coalesced; x is gathered through the read-only path
+// (27-point rows touch three x-planes, which stay L1/L2 resident).  The
+// reference's row-major ELLMatrix has its own kernel of this kind, whose groups
+// start aligned.
 // Epilogues: plain y = A x; y = A x with x.y (matvec_and_dot); and the CG
 // residual r = b - A x with r.r.  Dots accumulate in FP64 and reduce
 // deterministically (fixed grid, last block sums the block partials in order).
-// Matrices with rows longer than 32 entries use a warp-per-row kernel.
+// Matrices whose rows are stated to be longer than 32 entries, or are on
+// average, use a warp-per-row kernel.
 #include <algorithm>
 #include <climits>
 #include <cstdio>
@@ -35,8 +26,6 @@
 #include "mfe_internal.h"
 
 namespace mfe {
-
-constexpr int kMaxTileRowLen = 32;
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -52,7 +41,6 @@ struct SpmvParams {
   const T* __restrict__ x;
   T* __restrict__ y;
   const double* __restrict__ b;  // SPMV_RESID: y = b - A x
-  int cap;                       // elements per stage (multiple of 4)
   double* partials;
   unsigned* ticket;
   double* dot_out;  // used when cg == nullptr
@@ -136,146 +124,6 @@ __device__ __forceinline__ void spmv_epilogue(double total, CgState* cg, double*
   }
 }
 
-// A minimum of two blocks per SM in the launch bounds (shared memory allows
-// three or four) lets ptxas keep a row's gathers in flight at 96 registers
-// instead of 32-40: the 256^3 FP32 product 0.638 against 0.714 ms
-template <typename T, int ROWS, int S, int MODE>
-__global__ void __launch_bounds__(ROWS, 2) k_spmv_tiled(SpmvParams<T> P)
-{
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t bar[S];
-  __shared__ int64_t s_base_v[S], s_base_c[S];
-  __shared__ double red[32];
-  constexpr int VA = 16 / sizeof(T);  // values per 16 bytes
-  T* sv = reinterpret_cast<T*>(smem);
-  int32_t* sc = reinterpret_cast<int32_t*>(smem + (size_t)S * P.cap * sizeof(T));
-
-  const int tid = threadIdx.x;
-  const int64_t ntiles = (P.n + ROWS - 1) / ROWS;
-  if (tid == 0) {
-    for (int s = 0; s < S; ++s) mbar_init(&bar[s], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-
-  // producer (thread 0): stage nonzeros [a, e) of one tile into stage s
-  auto issue = [&](int64_t a, int64_t e, int s) {
-    const int64_t av = a & ~(int64_t)(VA - 1);
-    const int64_t ac = a & ~(int64_t)3;
-    int64_t bv = min((e + VA - 1) & ~(int64_t)(VA - 1), P.nnz & ~(int64_t)(VA - 1));
-    int64_t bc = min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3);
-    if (bv < av) bv = av;
-    if (bc < ac) bc = ac;
-    if (max(bv, e) - av > P.cap || max(bc, e) - ac > P.cap) {
-      // cannot happen when every row has <= max_len nonzeros (the host sizes
-      // cap from max_len); record it and stage nothing
-      atomicOr(P.err, ERR_TILE_OVERFLOW);
-      s_base_v[s] = a;
-      s_base_c[s] = a;
-      mbar_arrive_expect_tx(&bar[s], 0);
-      return;
-    }
-    s_base_v[s] = av;
-    s_base_c[s] = ac;
-    T* dv = sv + (size_t)s * P.cap;
-    int32_t* dc = sc + (size_t)s * P.cap;
-    // ragged tail past the last 16-byte boundary of the arrays: plain loads
-    for (int64_t k = bv; k < e; ++k) dv[k - av] = P.vals[k];
-    for (int64_t k = bc; k < e; ++k) dc[k - ac] = P.cols[k];
-    fence_proxy_async_smem();
-    const unsigned bytes_v = (unsigned)((bv - av) * sizeof(T));
-    const unsigned bytes_c = (unsigned)((bc - ac) * sizeof(int32_t));
-    mbar_arrive_expect_tx(&bar[s], bytes_v + bytes_c);
-    if (bytes_v) bulk_g2s(dv, P.vals + av, bytes_v, &bar[s]);
-    if (bytes_c) bulk_g2s(dc, P.cols + ac, bytes_c, &bar[s]);
-  };
-  auto tile_bounds = [&](int64_t t, int64_t& a, int64_t& e) {
-    a = __ldg(&P.ro[t * ROWS]);
-    e = __ldg(&P.ro[min(P.n, t * ROWS + ROWS)]);
-  };
-
-  if (tid == 0) {
-    for (int s = 0; s < S; ++s) {
-      const int64_t t = blockIdx.x + (int64_t)s * gridDim.x;
-      if (t < ntiles) {
-        int64_t a, e;
-        tile_bounds(t, a, e);
-        issue(a, e, s);
-      }
-    }
-  }
-
-  double dacc = 0.0;
-  int it = 0;
-  int64_t tile = blockIdx.x;
-  // row offsets of this thread's row in the current tile (prefetched)
-  int32_t ra = 0, rb = 0;
-  {
-    const int64_t r = tile * ROWS + tid;
-    if (tile < ntiles && r < P.n) {
-      ra = __ldg(&P.ro[r]);
-      rb = __ldg(&P.ro[r + 1]);
-    }
-  }
-  bool ok = true;
-  for (; tile < ntiles; tile += gridDim.x, ++it) {
-    const int s = it % S;
-    const unsigned parity = (unsigned)((it / S) & 1);
-    // prefetch the next tile's row offsets into registers
-    const int64_t ntile = tile + gridDim.x;
-    const int64_t nr = ntile * ROWS + tid;
-    int32_t na = 0, nb = 0;
-    if (ntile < ntiles && nr < P.n) {
-      na = __ldg(&P.ro[nr]);
-      nb = __ldg(&P.ro[nr + 1]);
-    }
-    // thread 0: bounds of the tile it will stage into s after this one
-    const int64_t itile = tile + (int64_t)S * gridDim.x;
-    int64_t ia = 0, ie = 0;
-    if (tid == 0 && itile < ntiles) tile_bounds(itile, ia, ie);
-    ok = mbar_wait_bounded(&bar[s], parity);
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    const int64_t r = tile * ROWS + tid;
-    if (r < P.n) {
-      const int len = rb - ra;
-      const T* rv = sv + (size_t)s * P.cap + (ra - s_base_v[s]);
-      const int32_t* rc = sc + (size_t)s * P.cap + (ra - s_base_c[s]);
-      const T sum = row_dot<T, 27>(rv, rc, len, P.x);
-      if (MODE == SPMV_RESID) {
-        const double rr = P.b[r] - (double)sum;
-        P.y[r] = (T)rr;
-        dacc = fma(rr, rr, dacc);
-      } else {
-        P.y[r] = sum;
-        if (MODE == SPMV_DOT) dacc = fma((double)sum, (double)__ldg(&P.x[r]), dacc);
-      }
-    }
-    ra = na;
-    rb = nb;
-    __syncthreads();  // every thread is done reading stage s
-    if (tid == 0 && itile < ntiles) issue(ia, ie, s);
-  }
-  if (!ok) {
-    if (tid == 0) {
-      atomicOr(P.err, ERR_WAIT_TIMEOUT);
-      // drain: give every stage that may still have copies in flight a
-      // bounded chance to complete before the block exits
-      for (int s = 0; s < S; ++s) {
-        const int j = it + s;
-        mbar_wait_bounded(&bar[j % S], (unsigned)((j / S) & 1));
-      }
-    }
-    return;
-  }
-  if (MODE != SPMV_PLAIN) {
-    const double bt = block_sum(dacc, red);
-    double total;
-    if (grid_reduce_last(bt, P.partials, P.ticket, red, &total) && tid == 0)
-      spmv_epilogue<MODE>(total, P.cg, P.dot_out);
-  }
-}
-
 // Warp-staged products: a warp per group of 32 rows, whose nonzeros are
 // contiguous in both layouts below (CSR: ro[32g] .. ro[32g+32]; the
 // reference's ELLMatrix: 32 g K .. 32 (g+1) K, short rows padded).  Lane 0
@@ -283,8 +131,7 @@ __global__ void __launch_bounds__(ROWS, 2) k_spmv_tiled(SpmvParams<T> P)
 // warp's own shared memory, with its own mbarrier (no block barrier in the
 // loop), and every lane sums rows from there.  The 256^3 FP64 CSR product took
 // 1.14 ms this way, two stages per warp, against 2.09 ms with 128-row tiles
-// behind block barriers (FP32 rows, half the bytes per stage, stay on the tiled
-// kernel).
+// behind block barriers.
 constexpr int kStgWarps = 2;    // warps per block
 constexpr int kStgMaxLen = 32;  // longer rows: the warp-per-row kernel
 
@@ -297,16 +144,17 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
   return ell ? 32 * max_len : ((32 * max_len + 8) + 3) & ~3;
 }
 
-// FP64 CSR rows.  A stage starts on the 16-byte boundaries at or below its
+// CSR rows.  A stage starts on the 16-byte boundaries at or below its
 // group's first nonzero, and the ragged end of the arrays arrives by plain
 // loads.  The stage is one per warp, of `cap` entries (the host's guess from the
 // mean row length): twenty-four warps per SM, a part of them computing while the
 // others' next groups arrive.  Groups that do not fit the stage, or hold a row
 // over kAnyLongest, read from global memory, a row at a time over the warp, so
 // the longest row need not be known.  `most`: what a group may take up when it is
-// (INT_MAX else); more is an error in the caller's max_row_len, and recorded.
+// (INT_MAX else); more is an error in the caller's max_row_len, and recorded (FP32:
+// of four groups together).
 //
-// What bounds it: the FP64 pipe, whose instructions take 17 clocks an SM whatever
+// What bounds it in FP64: the FP64 pipe, whose instructions take 17 clocks an SM whatever
 // the number of lanes at work.  Hence the rows in pairs (row_pair): 1.48 M rows
 // of 4 to 27 entries, 15.5 on average, take 18 FMAs a group instead of 27.
 // Measured there, us per call: a pass for the longest row, two stages and 27
@@ -314,7 +162,9 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // SM 86 / 79 / 76 (50 are the bytes at the HBM rate).  Rows of 27 entries (no
 // pairs): 126 / 106; of 3 to 7: 120 / 58; of 20 to 40: 682 / 273.  Cutting a
 // group's entries into 32 equal runs, a lane per run, took twice the
-// instructions, 147 us.
+// instructions, 147 us.  FP32 rows (no pairs) against 128-row tiles behind block
+// barriers: 1.48 M rows of 27 59 / 53, of 4 to 27 64 / 53, 12.3 M 445 / 410; without
+// the longest row's pass besides 85 / 53, and 15,625 rows 23 / 7.
 constexpr int kAnyLongest = 54;
 constexpr int kAnyBlocks = 12;  // per SM
 
@@ -386,8 +236,8 @@ __device__ __forceinline__ double pair_dot(const RowPair& q, int st, const doubl
   return mine + help;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<double> P, int cap, int most)
+template <typename T, int MODE>
+__global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<T> P, int cap, int most)
 {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t bar[kStgWarps];
@@ -395,9 +245,10 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
   __shared__ double red[32];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
-  const size_t vbytes = (size_t)cap * sizeof(double);
+  constexpr int VA = 16 / sizeof(T);
+  const size_t vbytes = (size_t)cap * sizeof(T);
   unsigned char* const stage = smem + (size_t)w * (vbytes + (size_t)cap * sizeof(int32_t));
-  double* const dv = reinterpret_cast<double*>(stage);
+  T* const dv = reinterpret_cast<T*>(stage);
   int32_t* const dc = reinterpret_cast<int32_t*>(stage + vbytes);
   const int64_t ngroups = (P.n + 31) / 32;
   const int64_t nw = (int64_t)gridDim.x * kStgWarps;
@@ -410,21 +261,30 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
 
   // up to 3 elements of slack at each end of a group (16-byte boundaries)
   auto staged = [&](int64_t a, int64_t e) { return e - a + 8 <= cap; };
+  // the ends of [a, e) on 16-byte boundaries, within the arrays
+  auto last = [&](int64_t from, int64_t e, int v) {
+    return max(from, min((e + v - 1) & ~(int64_t)(v - 1), P.nnz & ~(int64_t)(v - 1)));
+  };
+  // lane 0, when the longest row is stated: does group g keep to it?
+  auto check = [&](int64_t g) {
+    constexpr int kRows = sizeof(T) == 8 ? 32 : 128;
+    const int64_t r0 = g * 32 / kRows * kRows, a = __ldg(&P.ro[r0]), e = __ldg(&P.ro[min(P.n, r0 + kRows)]);
+    const int64_t av = a & ~(int64_t)(VA - 1), ac = a & ~(int64_t)3;
+    if (max(last(av, e, VA), e) - av > most || max(last(ac, e, 4), e) - ac > most)
+      atomicOr(P.err, ERR_TILE_OVERFLOW);
+  };
   // lane 0: nonzeros [a, e) of one group into the stage
   auto issue = [&](int64_t a, int64_t e) {
-    const int64_t av = a & ~(int64_t)1, ac = a & ~(int64_t)3;
-    const int64_t bv = max(av, min((e + 1) & ~(int64_t)1, P.nnz & ~(int64_t)1));
-    const int64_t bc = max(ac, min((e + 3) & ~(int64_t)3, P.nnz & ~(int64_t)3));
-    if (max(bv, e) - av > most || max(bc, e) - ac > most) atomicOr(P.err, ERR_TILE_OVERFLOW);
     if (!staged(a, e)) {
       mbar_arrive_expect_tx(&bar[w], 0);
       return;
     }
+    const int64_t av = a & ~(int64_t)(VA - 1), ac = a & ~(int64_t)3, bv = last(av, e, VA), bc = last(ac, e, 4);
     // ragged tail past the last 16-byte boundary of the arrays: plain loads
     for (int64_t k = bv; k < e; ++k) dv[k - av] = P.vals[k];
     for (int64_t k = bc; k < e; ++k) dc[k - ac] = P.cols[k];
     fence_proxy_async_smem();
-    const unsigned bytes_v = (unsigned)((bv - av) * sizeof(double));
+    const unsigned bytes_v = (unsigned)((bv - av) * sizeof(T));
     const unsigned bytes_c = (unsigned)((bc - ac) * sizeof(int32_t));
     mbar_arrive_expect_tx(&bar[w], bytes_v + bytes_c);
     if (bytes_v) bulk_g2s(dv, P.vals + av, bytes_v, &bar[w]);
@@ -455,20 +315,27 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
       st = (int)(__ldg(&P.ro[r]) - a);
       en = (int)(__ldg(&P.ro[r + 1]) - a);
     }
-    if (lane == 0 && gn < ngroups) bounds(gn, na, ne);
+    if (lane == 0) {
+      if (most != INT_MAX) check(g);
+      if (gn < ngroups) bounds(gn, na, ne);
+    }
     ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w], (unsigned)(it & 1), wait_ns));
     if (!ok) break;
-    double sum = 0.0;
+    T sum = T(0);
     if (staged(a, e) && __reduce_max_sync(0xffffffffu, en - st) <= kAnyLongest) {
-      const double* gv = dv + (a & 1);
+      const T* gv = dv + (a & (VA - 1));
       const int32_t* gc = dc + (a & 3);
-      const RowPair q = row_pair(st, en, lanes[w]);
-      if (__reduce_max_sync(0xffffffffu, q.own + q.extra) <= kPairSteps) sum = pair_dot(q, st, gv, gc, P.x);
-      else sum = row_dot<double, 27>(gv + st, gc + st, en - st, P.x);
+      if constexpr (sizeof(T) == 8) {
+        const RowPair q = row_pair(st, en, lanes[w]);
+        if (__reduce_max_sync(0xffffffffu, q.own + q.extra) <= kPairSteps) sum = pair_dot(q, st, gv, gc, P.x);
+        else sum = row_dot<T, 27>(gv + st, gc + st, en - st, P.x);
+      } else {
+        sum = row_dot<T, 27>(gv + st, gc + st, en - st, P.x);
+      }
     } else {
       for (int j = 0; j < 32; ++j) {
         const int js = __shfl_sync(0xffffffffu, st, j), je = __shfl_sync(0xffffffffu, en, j);
-        double v = 0.0;
+        T v = T(0);
         for (int k = js + lane; k < je; k += 32) v = fma(P.vals[a + k], __ldg(&P.x[P.cols[a + k]]), v);
         v = warp_sum(v);
         if (lane == j) sum = v;
@@ -476,12 +343,12 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
     }
     if (r < P.n) {
       if (MODE == SPMV_RESID) {
-        const double rr = P.b[r] - sum;
-        P.y[r] = rr;
+        const double rr = P.b[r] - (double)sum;
+        P.y[r] = (T)rr;
         dacc = fma(rr, rr, dacc);
       } else {
         P.y[r] = sum;
-        if (MODE == SPMV_DOT) dacc = fma(sum, __ldg(&P.x[r]), dacc);
+        if (MODE == SPMV_DOT) dacc = fma((double)sum, (double)__ldg(&P.x[r]), dacc);
       }
     }
     __syncwarp();  // every lane is done reading the stage
@@ -684,78 +551,6 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr int kStages = 2;
-
-// Rows per tile (= threads per CTA): 128 by default; MFE_SPMV_ROWS selects
-// 64 or 256 for launch-shape sweeps.
-static int tile_rows()
-{
-  static int rows = 0;
-  if (rows == 0) {
-    rows = 128;
-    if (const char* v = getenv("MFE_SPMV_ROWS")) {
-      const int r = atoi(v);
-      if (r == 64 || r == 128 || r == 256) rows = r;
-    }
-  }
-  return rows;
-}
-
-// Stage capacity (elements) for rows of at most max_len nonzeros: the tile's
-// nonzeros plus the 16-byte alignment slack at both ends, kept a multiple of 4
-// so every stage starts 16-byte aligned.
-static int tile_cap(int rows, int max_len)
-{
-  return ((rows * max_len + 8) + 3) & ~3;
-}
-
-template <typename T>
-static size_t tiled_smem(int rows, int max_len)
-{
-  return (size_t)kStages * tile_cap(rows, max_len) * (sizeof(T) + sizeof(int32_t));
-}
-
-template <typename T, int ROWS, int MODE>
-static cudaError_t configure_one()
-{
-  return cudaFuncSetAttribute(k_spmv_tiled<T, ROWS, kStages, MODE>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)tiled_smem<T>(ROWS, kMaxTileRowLen));
-}
-
-template <int ROWS>
-static cudaError_t configure_rows()
-{
-  cudaError_t e = configure_one<float, ROWS, SPMV_PLAIN>();
-  if (e == cudaSuccess) e = configure_one<float, ROWS, SPMV_DOT>();
-  return e;
-}
-
-// Shared-memory opt-in for every tiled instantiation, once per device (a
-// function attribute, so it is set before any stream capture uses them).
-static cudaError_t configure_tiled(int device)
-{
-  static bool done[64] = {};
-  if (device >= 0 && device < 64 && done[device]) return cudaSuccess;
-  cudaError_t e = configure_rows<64>();
-  if (e == cudaSuccess) e = configure_rows<128>();
-  if (e == cudaSuccess) e = configure_rows<256>();
-  if (e == cudaSuccess && device >= 0 && device < 64) done[device] = true;
-  return e;
-}
-
-// CTAs per SM for the tiled kernel (MFE_SPMV_CTAS_PER_SM overrides, for
-// launch-shape sweeps); limited by shared memory.
-static int tiled_ctas_per_sm(size_t smem)
-{
-  int per_sm = (int)((227 * 1024) / (smem + 1024));
-  if (const char* v = getenv("MFE_SPMV_CTAS_PER_SM")) {
-    const int o = atoi(v);
-    if (o > 0 && o < per_sm) per_sm = o;
-  }
-  return std::max(1, per_sm);
-}
-
 // ---- warp-staged kernels ----
 mfe_status take_wait_injection(mfe_ctx* ctx, uint64_t* withhold_ns)
 {
@@ -808,23 +603,28 @@ static int any_cap(int64_t n, int64_t nnz, int max_len)
   return stg_cap(std::max(1, std::min(most, (int)(1.25 * (double)nnz / (double)std::max<int64_t>(n, 1)) + 2)), false);
 }
 
-static size_t any_smem(int cap) { return (size_t)kStgWarps * cap * (sizeof(double) + sizeof(int32_t)); }
+template <typename T>
+static size_t any_smem(int cap)
+{
+  return (size_t)kStgWarps * cap * (sizeof(T) + sizeof(int32_t));
+}
 
+template <typename T>
 static int any_grid(mfe_ctx* ctx, int64_t nrows, int cap)
 {
-  const int per_sm = std::max(1, std::min(kAnyBlocks, (int)((228 * 1024) / (any_smem(cap) + 1024 + 512))));
+  const int per_sm = std::max(1, std::min(kAnyBlocks, (int)((228 * 1024) / (any_smem<T>(cap) + 1024 + 512))));
   return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)kStgWarps),
                                                      (int64_t)ctx->sm_count * per_sm));
 }
 
-template <int MODE>
-static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<double>& P, int max_len)
+template <typename T, int MODE>
+static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<T>& P, int max_len)
 {
   static bool configured[64] = {};
-  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<MODE>, any_smem(stg_cap(kStgMaxLen, false)), configured));
+  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<T, MODE>, any_smem<T>(stg_cap(kStgMaxLen, false)), configured));
   const int cap = any_cap(P.n, P.nnz, max_len);
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
-  k_spmv_any<MODE><<<any_grid(ctx, P.n, cap), kStgWarps * 32, any_smem(cap), ctx->stream>>>(
+  k_spmv_any<T, MODE><<<any_grid<T>(ctx, P.n, cap), kStgWarps * 32, any_smem<T>(cap), ctx->stream>>>(
       P, cap, max_len > 0 ? stg_cap(max_len, false) : INT_MAX);
   return check_launch(ctx, "k_spmv_any");
 }
@@ -835,13 +635,8 @@ int spmv_grid(mfe_ctx* ctx, const mfe_csr* A)
   if (max_len > kStgMaxLen)  // the warp-per-row kernel
     return (int)std::max<int64_t>(
         1, std::min<int64_t>(ceil_div(A->nrows * 32, 256), (int64_t)ctx->sm_count * 8));
-  if (A->dtype == MFE_F64) {
-    return any_grid(ctx, A->nrows, any_cap(A->nrows, A->nnz, A->max_row_len));
-  }
-  const int rows = tile_rows();
-  const int64_t ntiles = ceil_div(A->nrows, rows);
-  const int per_sm = tiled_ctas_per_sm(tiled_smem<float>(rows, max_len));
-  return (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)ctx->sm_count * per_sm));
+  const int cap = any_cap(A->nrows, A->nnz, A->max_row_len);
+  return A->dtype == MFE_F64 ? any_grid<double>(ctx, A->nrows, cap) : any_grid<float>(ctx, A->nrows, cap);
 }
 
 mfe_status ensure_max_row_len(mfe_ctx* ctx, const mfe_csr* A, int* max_len)
@@ -877,8 +672,6 @@ static mfe_status launch_t(mfe_ctx* ctx, const mfe_csr* A, const T* x, T* y, con
   P.x = x;
   P.y = y;
   P.b = b;
-  const int rows = tile_rows();
-  P.cap = tile_cap(rows, std::max(max_len, 1));
   P.partials = sink ? sink->partials : nullptr;
   P.ticket = sink ? sink->ticket : nullptr;
   P.dot_out = sink ? sink->out : nullptr;
@@ -888,24 +681,8 @@ static mfe_status launch_t(mfe_ctx* ctx, const mfe_csr* A, const T* x, T* y, con
   if (!P.err) return fail(ctx, MFE_OOM, "workspace allocation failed");
   if (cg) P.err = &cg->err;
   if (A->nrows == 0) return MFE_OK;
-  if (max_len <= kStgMaxLen && aligned16(A->vals) && aligned16(A->cols)) {
-    if constexpr (sizeof(T) == 8) {
-      return launch_any<MODE>(ctx, P, max_len);
-    } else {
-      MFE_CUDA_TRY(ctx, configure_tiled(ctx->device));
-      const size_t smem = tiled_smem<T>(rows, std::max(max_len, 1));
-      const int64_t ntiles = ceil_div(A->nrows, rows);
-      const int grid = (int)std::max<int64_t>(
-          1, std::min<int64_t>(ntiles, (int64_t)ctx->sm_count * tiled_ctas_per_sm(smem)));
-      if (rows == 64)
-        k_spmv_tiled<T, 64, kStages, MODE><<<grid, 64, smem, ctx->stream>>>(P);
-      else if (rows == 256)
-        k_spmv_tiled<T, 256, kStages, MODE><<<grid, 256, smem, ctx->stream>>>(P);
-      else
-        k_spmv_tiled<T, 128, kStages, MODE><<<grid, 128, smem, ctx->stream>>>(P);
-      return check_launch(ctx, "k_spmv_tiled");
-    }
-  }
+  if (max_len <= kStgMaxLen && aligned16(A->vals) && aligned16(A->cols))
+    return launch_any<T, MODE>(ctx, P, max_len);
   const int grid = (int)std::max<int64_t>(
       1, std::min<int64_t>(ceil_div(A->nrows * 32, 256), (int64_t)ctx->sm_count * 8));
   k_spmv_warp<T, MODE><<<grid, 256, 0, ctx->stream>>>(P);
@@ -919,14 +696,9 @@ mfe_status launch_spmv(mfe_ctx* ctx, const mfe_csr* A, const void* x, void* y,
   if (csr_is_box(A) && aligned16(A->vals) && aligned16(x) &&
       getenv("MFE_SPMV_GENERIC") == nullptr)
     return launch_spmv_box(ctx, A, x, y, sink, resid_b, cg_state);
-  // the longest row decides the kernel; FP64 rows of a mean length within the
-  // staged kernels' need not have it found first (k_spmv_any)
+  // the longest row where it is stated, else the mean, decides the kernel
   int max_len = A->max_row_len;
-  if (A->dtype == MFE_F64 && max_len <= 0) {
-    if (A->nnz > (int64_t)kStgMaxLen * A->nrows) max_len = kStgMaxLen + 1;
-  } else {
-    MFE_TRY(ensure_max_row_len(ctx, A, &max_len));
-  }
+  if (max_len <= 0 && A->nnz > (int64_t)kStgMaxLen * A->nrows) max_len = kStgMaxLen + 1;
   CgState* cg = static_cast<CgState*>(cg_state);
   if (A->dtype == MFE_F64) {
     const double* xd = static_cast<const double*>(x);
@@ -961,7 +733,6 @@ static mfe_status launch_ell_ns(mfe_ctx* ctx, const mfe_ell* E, const T* x, T* y
   P.x = x;
   P.y = y;
   P.b = b;
-  P.cap = stg_cap(E->ncols_per_row, true);
   P.partials = sink ? sink->partials : nullptr;
   P.ticket = sink ? sink->ticket : nullptr;
   P.dot_out = sink ? sink->out : nullptr;

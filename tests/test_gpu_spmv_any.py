@@ -1,11 +1,11 @@
-"""FP64 products with CSR rows of any lengths (k_spmv_any): rows in pairs and alone,
+"""Products with CSR rows of any lengths (k_spmv_any): rows in pairs and alone,
 empty rows, groups of 32 rows larger than the stage, long rows among short ones,
 the last partial group, and the dot's epilogue.
 
 Bound: each row is at most its length in FMAs plus the additions that join its
 partial sums (32 at most), every rounding at most 2^-53 of the sum of |a||x| so far:
 (len + 32) 2^-53 sum |a||x| against the same sum in extended precision (whose
-own rounding is 2^-11 of that)."""
+own rounding is 2^-11 of that).  FP32 rows the same with 2^-24."""
 import numpy as np
 import pytest
 
@@ -58,6 +58,27 @@ def test_uneven_rows(shape, n):
         d = M.matvec_and_dot(A, dev[3], y)
         yy = y.cpu().numpy()
         assert abs(d - float(np.dot(yy.astype(np.longdouble), x))) <= (n + 64) * 2.0**-53 * float(np.abs(yy * x).sum())
+
+
+@pytest.mark.parametrize("n", [33, 20011])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_uneven_rows_f32(shape, n):
+    rng = np.random.default_rng(4)
+    lens = SHAPES[shape](rng, n).astype(np.int64)
+    ro = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = rng.integers(0, n, ro[-1]).astype(np.int32)
+    vals, x = (rng.normal(size=k).astype(np.float32) for k in (ro[-1], n))
+    dev = [torch.from_numpy(a).cuda() for a in (ro, np.append(cols, [0] * 4).astype(np.int32),
+                                                np.append(vals, np.zeros(4, np.float32)), x)]
+    A = M.CSRMatrix(dev[0], dev[1][:ro[-1]], dev[2][:ro[-1]])
+    y = torch.full((n,), 7.0, dtype=torch.float32, device="cuda")
+    M.matvec(A, dev[3], y)
+    prod = vals.astype(np.float64) * x[cols].astype(np.float64)
+    rows = np.repeat(np.arange(n), lens)
+    exact, size = np.zeros(n), np.zeros(n)
+    np.add.at(exact, rows, prod)
+    np.add.at(size, rows, np.abs(prod))
+    assert (np.abs(y.cpu().numpy() - exact) <= (lens + 32) * 2.0**-24 * size).all()
 
 
 @pytest.mark.parametrize("stated,refused", [(27, False), (26, False), (25, True), (4, True)])
