@@ -163,8 +163,9 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // pairs): 126 / 106; of 3 to 7: 120 / 58; of 20 to 40: 682 / 273.  Cutting a
 // group's entries into 32 equal runs, a lane per run, took twice the
 // instructions, 147 us.  FP32 rows (no pairs) against 128-row tiles behind block
-// barriers: 1.48 M rows of 27 59 / 53, of 4 to 27 64 / 53, 12.3 M 445 / 410; without
-// the longest row's pass besides 85 / 53, and 15,625 rows 23 / 7.
+// barriers, 1.48 M rows of 27 / of 4 to 27 / 12.3 M rows of 27: longest row stated
+// 59, 64, 445 before and 57, 58, 425 now; not stated (a pass for it before) 83,
+// 85, 475 and 55, 55, 405; 15,625 rows 23 and 8.
 constexpr int kAnyLongest = 54;
 constexpr int kAnyBlocks = 12;  // per SM
 
