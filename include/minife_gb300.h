@@ -63,7 +63,7 @@ typedef struct mfe_csr {
   int32_t* cols;        /* device, nnz */
   void* vals;           /* device, nnz of dtype */
   int32_t dtype;        /* mfe_dtype */
-  int32_t max_row_len;  /* 0 = unknown (computed on first use) */
+  int32_t max_row_len;  /* 0 = unknown (a product goes by the mean, a solve finds it) */
   /* box the matrix was assembled on (0 if not an assembled box); lets the
    * solver use the 27-point stencil layout of those rows */
   int32_t box_nx, box_ny, box_nz;

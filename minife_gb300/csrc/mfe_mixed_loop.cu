@@ -211,7 +211,8 @@ mfe_status launch_mixed_loop(mfe_ctx* ctx, const mfe_csr* A, const float* coef, 
   P.Nz = A->box_nz + 1;
   P.Nxp = stencil_pitch(A);
   P.NP = P.Nxp * P.Ny;
-  if (!stencil_mirror_classes(coef, P.w)) return fail(ctx, MFE_NOT_SUPPORTED, "the loop takes mirror-symmetric stencils");
+  if (!stencil_mirror_classes(coef, P.w))
+    return fail(ctx, MFE_NOT_SUPPORTED, "the loop takes mirror-symmetric stencils");
   P.dd = coef[27];
   double* ws = static_cast<double*>(workspace(ctx, "mixed.loop", sizeof(double) * 4096 + 16));
   if (!ws) return fail(ctx, MFE_OOM, "mixed solver workspace allocation failed");
