@@ -989,7 +989,7 @@ __global__ void __launch_bounds__(kBxVT)
                 const V* __restrict__ Ap)
 {
   __shared__ double red[32];
-  __shared__ float2 redf[32];
+  __shared__ float redf[32][3];
   __shared__ bool last;
   const int cnt = *Q.count;
   if (cnt == 0) return;
@@ -1042,14 +1042,13 @@ __global__ void __launch_bounds__(kBxVT)
       else
         acc = fma(rn, rn, acc);
     }
-    // FP32: double-float until one number per block is left (the FP64 sums of
+    // FP32 operations until one number per block is left (the FP64 sums of
     // every warp queued on the FP64 pipe: 24 boxes of 16 to 96 18.7 us, now 16.0)
     double bt;
     if constexpr (kX) {
       bt = block_sum(acc, red);
     } else {
-      block_sum_df(facc.hi, facc.lo, redf);
-      bt = facc.value();
+      bt = block_sum_tf(facc, redf).value();
     }
     if (threadIdx.x == 0) {
       Q.chunk_part[d.chunk_base + lc] = bt;

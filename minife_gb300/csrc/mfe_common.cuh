@@ -284,6 +284,58 @@ __device__ __forceinline__ void block_sum_df(float& hi, float& lo, float2* scrat
   }
 }
 
+// Sums of double-float pairs with FP32 operations to more bits than FP64 keeps
+// (three floats; what is rounded lies 2^-72 below the largest term): the FP64
+// pipe is left with the two additions that make a double of one sum.
+struct TFSum {
+  float h = 0.0f, m = 0.0f, l = 0.0f;
+  // a += b, the rounding error returned (TwoSum)
+  __device__ __forceinline__ static float two_sum(float& a, float b)
+  {
+    const float t = __fadd_rn(a, b);
+    const float bp = __fsub_rn(t, a);
+    const float err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, bp)), __fsub_rn(b, bp));
+    a = t;
+    return err;
+  }
+  __device__ __forceinline__ void add(float hi, float lo, float ll = 0.0f)
+  {
+    const float e1 = two_sum(h, hi), e2 = two_sum(m, lo), e3 = two_sum(m, e1);
+    l = __fadd_rn(l, __fadd_rn(ll, __fadd_rn(e2, e3)));
+  }
+  __device__ __forceinline__ double value() const { return f2d_exact(h) + (f2d_exact(m) + f2d_exact(l)); }
+};
+
+// the block's sum, valid in thread 0; scratch: three floats for each warp
+__device__ __forceinline__ TFSum block_sum_tf(const DFAcc& a, float (*scratch)[3])
+{
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  TFSum s;
+  s.add(a.hi, a.lo);
+  auto warp = [&] {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float h = __shfl_xor_sync(0xffffffffu, s.h, o), m = __shfl_xor_sync(0xffffffffu, s.m, o),
+                  l = __shfl_xor_sync(0xffffffffu, s.l, o);
+      s.add(h, m, l);
+    }
+  };
+  warp();
+  __syncthreads();  // scratch may be reused across calls
+  if (lane == 0) {
+    scratch[wid][0] = s.h;
+    scratch[wid][1] = s.m;
+    scratch[wid][2] = s.l;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    s = TFSum{};
+    if (lane < (int)(blockDim.x + 31) >> 5) s.add(scratch[lane][0], scratch[lane][1], scratch[lane][2]);
+    warp();
+  }
+  return s;
+}
+
 // grid_reduce_last on double-float pairs: each block's pair goes to its
 // 8-byte slot of partials, the last block sums them in block order and thread
 // 0 gets hi + lo in FP64 (the one FP64 operation).

@@ -1027,17 +1027,17 @@ __global__ void __launch_bounds__(kVT)
     }
   }
   // entry VW*t + c holds right-hand side (VW*t + c) % nrhs; entries t + k*kVT
-  // share thread t's right-hand side t % nrhs.  The double-float sums stay so
-  // until one number per thread is left: eleven FP64 additions per thread here
-  // cost a 64^3 x 32 solve 2.2 us per iteration.
+  // share thread t's right-hand side t % nrhs.  The double-float sums are added
+  // in FP32 operations until one number per thread is left (eleven FP64 additions
+  // per thread cost a 64^3 x 32 solve 2.2 us per iteration).
   double a = 0.0;
   if constexpr (sizeof(V) == 4) {
 #pragma unroll
     for (int c = 0; c < VW; ++c) ent[VW * threadIdx.x + c] = make_float2(facc[c].hi, facc[c].lo);
     __syncthreads();
-    DFAcc t;
+    TFSum t;
 #pragma unroll
-    for (int k = 0; k < VW; ++k) df_add(t.hi, t.lo, ent[threadIdx.x + k * kVT].x, ent[threadIdx.x + k * kVT].y);
+    for (int k = 0; k < VW; ++k) t.add(ent[threadIdx.x + k * kVT].x, ent[threadIdx.x + k * kVT].y);
     a = t.value();
   } else {
 #pragma unroll
