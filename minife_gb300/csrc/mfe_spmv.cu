@@ -150,9 +150,9 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // mean row length): twenty-four warps per SM, a part of them computing while the
 // others' next groups arrive.  Groups that do not fit the stage, or hold a row
 // over kAnyLongest, read from global memory, a row at a time over the warp, so
-// the longest row need not be known.  `most`: what a group may take up when it is
-// (INT_MAX else); more is an error in the caller's max_row_len, and recorded (FP32:
-// of four groups together).
+// the longest row need not be known.  `most`: what kCheckRows rows may take up when
+// it is stated (INT_MAX else); more is an error in the caller's max_row_len, and
+// recorded.
 //
 // What bounds it in FP64: the FP64 pipe, whose instructions take 17 clocks an SM whatever
 // the number of lanes at work.  Hence the rows in pairs (row_pair): 1.48 M rows
@@ -168,6 +168,12 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // 85, 475 and 55, 55, 405; 15,625 rows 23 and 8.
 constexpr int kAnyLongest = 54;
 constexpr int kAnyBlocks = 12;  // per SM
+
+// rows whose entries together are held against a stated longest row, and what they
+// may take up with the rounding to 16 bytes
+template <typename T>
+constexpr int kCheckRows = sizeof(T) == 8 ? 32 : 128;
+constexpr int stated_most(int rows, int max_len) { return (rows * max_len + 8 + 3) & ~3; }
 
 // A group's 32 rows shared out in pairs: the lanes ranked by row length, the
 // r-th shortest row's lane also takes the end of the r-th longest, so that both
@@ -266,10 +272,14 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
   auto last = [&](int64_t from, int64_t e, int v) {
     return max(from, min((e + v - 1) & ~(int64_t)(v - 1), P.nnz & ~(int64_t)(v - 1)));
   };
-  // lane 0, when the longest row is stated: does group g keep to it?
-  auto check = [&](int64_t g) {
-    constexpr int kRows = sizeof(T) == 8 ? 32 : 128;
-    const int64_t r0 = g * 32 / kRows * kRows, a = __ldg(&P.ro[r0]), e = __ldg(&P.ro[min(P.n, r0 + kRows)]);
+  // lane 0, when the longest row is stated: do the kCheckRows<T> rows around group
+  // g, nonzeros [a, e), keep to it?
+  auto check = [&](int64_t g, int64_t a, int64_t e) {
+    if constexpr (kCheckRows<T> != 32) {
+      const int64_t r0 = g * 32 / kCheckRows<T> * kCheckRows<T>;
+      a = __ldg(&P.ro[r0]);
+      e = __ldg(&P.ro[min(P.n, r0 + kCheckRows<T>)]);
+    }
     const int64_t av = a & ~(int64_t)(VA - 1), ac = a & ~(int64_t)3;
     if (max(last(av, e, VA), e) - av > most || max(last(ac, e, 4), e) - ac > most)
       atomicOr(P.err, ERR_TILE_OVERFLOW);
@@ -317,7 +327,7 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
       en = (int)(__ldg(&P.ro[r + 1]) - a);
     }
     if (lane == 0) {
-      if (most != INT_MAX) check(g);
+      if (most != INT_MAX) check(g, a, e);
       if (gn < ngroups) bounds(gn, na, ne);
     }
     ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w], (unsigned)(it & 1), wait_ns));
@@ -626,7 +636,7 @@ static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<T>& P, int max_len)
   const int cap = any_cap(P.n, P.nnz, max_len);
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
   k_spmv_any<T, MODE><<<any_grid<T>(ctx, P.n, cap), kStgWarps * 32, any_smem<T>(cap), ctx->stream>>>(
-      P, cap, max_len > 0 ? stg_cap(max_len, false) : INT_MAX);
+      P, cap, max_len > 0 ? stated_most(kCheckRows<T>, max_len) : INT_MAX);
   return check_launch(ctx, "k_spmv_any");
 }
 
