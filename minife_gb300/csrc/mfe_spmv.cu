@@ -148,24 +148,30 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // group's first nonzero, and the ragged end of the arrays arrives by plain
 // loads.  The stage is one per warp, of `cap` entries (the host's guess from the
 // mean row length): twenty-four warps per SM, a part of them computing while the
-// others' next groups arrive.  Groups that do not fit the stage, or hold a row
-// over kAnyLongest, read from global memory, a row at a time over the warp, so
-// the longest row need not be known.  `most`: what kCheckRows rows may take up when
-// it is stated (INT_MAX else); more is an error in the caller's max_row_len, and
-// recorded.
+// others' next groups arrive.  A group that does not fit the stage, or holds a row
+// over kAnyLongest, is taken in parts of 16, 8, ... 1 rows with 2, 4, ... 32 lanes
+// a row, through the stage as long as a part fits it, so the longest row need not
+// be known.  `most`: what kCheckRows rows may take up when it is stated (INT_MAX
+// else); more is an error in the caller's max_row_len, and recorded.
 //
 // What bounds it in FP64: the FP64 pipe, whose instructions take 17 clocks an SM whatever
 // the number of lanes at work.  Hence the rows in pairs (row_pair): 1.48 M rows
 // of 4 to 27 entries, 15.5 on average, take 18 FMAs a group instead of 27.
 // Measured there, us per call: a pass for the longest row, two stages and 27
-// FMAs 121; without the pass 107; in pairs 103; one stage, 8 / 10 / 12 blocks per
+// FMAs 121; without the pass 107; in pairs 103; one stage, 16 / 20 / 24 warps per
 // SM 86 / 79 / 76 (50 are the bytes at the HBM rate).  Rows of 27 entries (no
-// pairs): 126 / 106; of 3 to 7: 120 / 58; of 20 to 40: 682 / 273.  Cutting a
+// pairs): 135 / 111; of 5: 126 / 69; of 20 to 40: 700 / 144.  Cutting a
 // group's entries into 32 equal runs, a lane per run, took twice the
 // instructions, 147 us.  FP32 rows (no pairs) against 128-row tiles behind block
-// barriers, 1.48 M rows of 27 / of 4 to 27 / 12.3 M rows of 27: longest row stated
-// 59, 64, 445 before and 57, 58, 425 now; not stated (a pass for it before) 83,
-// 85, 475 and 55, 55, 405; 15,625 rows 23 and 8.
+// barriers, 1.48 M rows of 27 / of 4 to 27: longest row stated 68, 65 before and
+// 63, 60 now; not stated (a pass for it before) 94, 90 and 63, 59.
+// Rows whose lengths come in regions (half of them 4 to 7, half 27 to 32, so that
+// every group of the second half is larger than the stage), FP64 / FP32: with the
+// longest row known and a stage for it 133 / 73; such groups a row at a time over
+// the warp 342 / 371; in parts 98 / 71.  Rows of 8 and 56 in turn 737 / 262 (a warp
+// per row), 714 / 663 (a row at a time), 254 / 128; one row of 200 among 31 of 10 930
+// / 465, 585 / 653, 317 / 111.  One row of 200,000 among rows of 20 takes 2990 / 1706
+// (a warp per row), 990 / 550.
 constexpr int kAnyLongest = 54;
 constexpr int kAnyBlocks = 12;  // per SM
 
@@ -243,6 +249,31 @@ __device__ __forceinline__ double pair_dot(const RowPair& q, int st, const doubl
   return mine + help;
 }
 
+// entries k, k + L, ... below end of a row times x; gv, gc: the values and columns;
+// any: an entry of the warp's rows (loaded in place of one past a row's end)
+template <typename T>
+__device__ __forceinline__ T strided_dot(const T* gv, const int32_t* gc, int k, int end, int L, int any,
+                                         const T* __restrict__ x)
+{
+  constexpr int kBatch = 9;  // gathers in flight
+  T s = T(0);
+  for (; __any_sync(0xffffffffu, k < end); k += kBatch * L) {
+    T v[kBatch], xv[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int at = k + i * L < end ? k + i * L : any;
+      xv[i] = ld_gather(&x[gc[at]]);
+      v[i] = gv[at];
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const T t = fma(v[i], xv[i], s);
+      s = k + i * L < end ? t : s;
+    }
+  }
+  return s;
+}
+
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<T> P, int cap, int most)
 {
@@ -314,8 +345,13 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
   const uint64_t wait_ns = P.withhold_ns ? P.withhold_ns : kWaitLimitNs;
   double dacc = 0.0;
   bool ok = true;
-  int it = 0;
-  for (int64_t g = g0; g < ngroups; g += nw, ++it) {
+  unsigned phase = 0;  // copies that have landed
+  auto landed = [&] {
+    const bool there = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w], phase & 1u, wait_ns));
+    if (there) ++phase;
+    return there;
+  };
+  for (int64_t g = g0; g < ngroups; g += nw) {
     const int64_t r = g * 32 + lane;
     const int64_t gn = g + nw;  // the group the stage takes next
     int64_t a, e, na = 0, ne = 0;
@@ -330,10 +366,12 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
       if (most != INT_MAX) check(g, a, e);
       if (gn < ngroups) bounds(gn, na, ne);
     }
-    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[w], (unsigned)(it & 1), wait_ns));
+    ok = landed();
     if (!ok) break;
     T sum = T(0);
-    if (staged(a, e) && __reduce_max_sync(0xffffffffu, en - st) <= kAnyLongest) {
+    const bool whole = staged(a, e);
+    const int longest = __reduce_max_sync(0xffffffffu, en - st);
+    if (whole && longest <= kAnyLongest) {
       const T* gv = dv + (a & (VA - 1));
       const int32_t* gc = dc + (a & 3);
       if constexpr (sizeof(T) == 8) {
@@ -344,13 +382,38 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
         sum = row_dot<T, 27>(gv + st, gc + st, en - st, P.x);
       }
     } else {
-      for (int j = 0; j < 32; ++j) {
-        const int js = __shfl_sync(0xffffffffu, st, j), je = __shfl_sync(0xffffffffu, en, j);
-        T v = T(0);
-        for (int k = js + lane; k < je; k += 32) v = fma(P.vals[a + k], __ldg(&P.x[P.cols[a + k]]), v);
-        v = warp_sum(v);
-        if (lane == j) sum = v;
+      // R rows at a time, L lanes a row: as few lanes as leave 27 entries to each
+      // and let the R rows fit the stage
+      int L = 2;
+      for (; L < 32; L *= 2) {
+        const int R = 32 / L;
+        const int lo = __shfl_sync(0xffffffffu, st, lane & ~(R - 1)), hi = __shfl_sync(0xffffffffu, en, lane | (R - 1));
+        if (__all_sync(0xffffffffu, en - st <= 27 * L && (whole || staged(lo, hi)))) break;
       }
+      const int R = 32 / L;
+      for (int j = 0; j < L; ++j) {
+        const int lo = __shfl_sync(0xffffffffu, st, j * R), hi = __shfl_sync(0xffffffffu, en, j * R + R - 1);
+        const int of = j * R + lane / L;
+        const int rs = __shfl_sync(0xffffffffu, st, of) + (lane & (L - 1)), re = __shfl_sync(0xffffffffu, en, of);
+        T v;
+        if (whole) {
+          v = strided_dot(dv + (a & (VA - 1)), dc + (a & 3), rs, re, L, lo, P.x);
+        } else if (staged(lo, hi)) {
+          __syncwarp();  // every lane is done reading the stage
+          if (lane == 0) issue(a + lo, a + hi);
+          ok = landed();
+          if (!ok) break;
+          v = strided_dot(dv + ((a + lo) & (VA - 1)) - lo, dc + ((a + lo) & 3) - lo, rs, re, L, lo, P.x);
+        } else {
+          // one row, longer than the stage
+          v = T(0);
+          for (int k = rs; k < re; k += 32) v = fma(P.vals[a + k], __ldg(&P.x[P.cols[a + k]]), v);
+        }
+        for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const T mine = __shfl_sync(0xffffffffu, v, (lane & (R - 1)) * L);
+        if (lane / R == j) sum = mine;
+      }
+      if (!ok) break;
     }
     if (r < P.n) {
       if (MODE == SPMV_RESID) {
@@ -370,7 +433,7 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
       atomicOr(P.err, ERR_WAIT_TIMEOUT);
       // drain: give the copy a bounded chance to land before the block exits (an
       // injected fault issued none)
-      if (P.withhold_ns == 0) mbar_wait_bounded(&bar[w], (unsigned)(it & 1));
+      if (P.withhold_ns == 0) mbar_wait_bounded(&bar[w], phase & 1u);
     }
     __syncwarp();
   }
