@@ -173,7 +173,7 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // / 465, 585 / 653, 317 / 111.  One row of 200,000 among rows of 20 takes 2990 / 1706
 // (a warp per row), 990 / 550.
 constexpr int kAnyLongest = 54;
-constexpr int kAnyBlocks = 12;  // per SM
+constexpr int kAnyWarps = 24;  // per SM, in blocks of W
 
 // rows whose entries together are held against a stated longest row, and what they
 // may take up with the rounding to 16 bytes
@@ -274,12 +274,12 @@ __device__ __forceinline__ T strided_dot(const T* gv, const int32_t* gc, int k, 
   return s;
 }
 
-template <typename T, int MODE>
-__global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvParams<T> P, int cap, int most)
+template <typename T, int MODE, int W>
+__global__ void __launch_bounds__(W * 32, kAnyWarps / W) k_spmv_any(SpmvParams<T> P, int cap, int most)
 {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t bar[kStgWarps];
-  __shared__ uint8_t lanes[kStgWarps][32];
+  __shared__ uint64_t bar[W];
+  __shared__ uint8_t lanes[W][32];
   __shared__ double red[32];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(kStgWarps * 32, kAnyBlocks) k_spmv_any(SpmvPar
   T* const dv = reinterpret_cast<T*>(stage);
   int32_t* const dc = reinterpret_cast<int32_t*>(stage + vbytes);
   const int64_t ngroups = (P.n + 31) / 32;
-  const int64_t nw = (int64_t)gridDim.x * kStgWarps;
-  const int64_t g0 = (int64_t)blockIdx.x * kStgWarps + w;
+  const int64_t nw = (int64_t)gridDim.x * W;
+  const int64_t g0 = (int64_t)blockIdx.x * W + w;
   if (lane == 0) {
     mbar_init(&bar[w], 1);
     fence_mbar_init();
@@ -677,30 +677,52 @@ static int any_cap(int64_t n, int64_t nnz, int max_len)
   return stg_cap(std::max(1, std::min(most, (int)(1.25 * (double)nnz / (double)std::max<int64_t>(n, 1)) + 2)), false);
 }
 
+// Warps per block.  A block's warps take neighbouring groups, whose rows mostly
+// read the same part of x: FP32 rows of columns within 3,000 of the diagonal, whose
+// large stages leave little L1, 600,000 rows of 27 to 32 / 20 to 32 / 27 entries,
+// blocks of two 119, 113, 110 us, of eight 93, 85, 87 (with columns within 30 even).
+// FP64 rows and short ones keep two (1.48 M FP64 rows of 4 to 27: 75.6 and 77.6).
 template <typename T>
-static size_t any_smem(int cap)
+static int any_warps(int cap)
 {
-  return (size_t)kStgWarps * cap * (sizeof(T) + sizeof(int32_t));
+  return sizeof(T) == 4 && cap > 25 * 32 ? 8 : 2;  // a mean row of 19 entries or more
+}
+
+template <typename T>
+static size_t any_smem(int cap, int warps)
+{
+  return (size_t)warps * cap * (sizeof(T) + sizeof(int32_t));
 }
 
 template <typename T>
 static int any_grid(mfe_ctx* ctx, int64_t nrows, int cap)
 {
-  const int per_sm = std::max(1, std::min(kAnyBlocks, (int)((228 * 1024) / (any_smem<T>(cap) + 1024 + 512))));
-  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)kStgWarps),
+  const int W = any_warps<T>(cap);
+  const int per_sm = std::max(1, std::min(kAnyWarps / W, (int)((228 * 1024) / (any_smem<T>(cap, W) + 1024 + 256 * W))));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)W),
                                                      (int64_t)ctx->sm_count * per_sm));
+}
+
+template <typename T, int MODE, int W>
+static mfe_status launch_any_w(mfe_ctx* ctx, SpmvParams<T>& P, int cap, int most)
+{
+  static bool configured[64] = {};
+  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<T, MODE, W>, any_smem<T>(stg_cap(kStgMaxLen, false), W),
+                           configured));
+  k_spmv_any<T, MODE, W><<<any_grid<T>(ctx, P.n, cap), W * 32, any_smem<T>(cap, W), ctx->stream>>>(P, cap, most);
+  return check_launch(ctx, "k_spmv_any");
 }
 
 template <typename T, int MODE>
 static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<T>& P, int max_len)
 {
-  static bool configured[64] = {};
-  MFE_TRY(staged_configure(ctx, (const void*)k_spmv_any<T, MODE>, any_smem<T>(stg_cap(kStgMaxLen, false)), configured));
   const int cap = any_cap(P.n, P.nnz, max_len);
+  const int most = max_len > 0 ? stated_most(kCheckRows<T>, max_len) : INT_MAX;
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
-  k_spmv_any<T, MODE><<<any_grid<T>(ctx, P.n, cap), kStgWarps * 32, any_smem<T>(cap), ctx->stream>>>(
-      P, cap, max_len > 0 ? stated_most(kCheckRows<T>, max_len) : INT_MAX);
-  return check_launch(ctx, "k_spmv_any");
+  if constexpr (sizeof(T) == 4) {
+    if (any_warps<T>(cap) == 8) return launch_any_w<T, MODE, 8>(ctx, P, cap, most);
+  }
+  return launch_any_w<T, MODE, 2>(ctx, P, cap, most);
 }
 
 int spmv_grid(mfe_ctx* ctx, const mfe_csr* A)
