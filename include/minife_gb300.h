@@ -248,6 +248,13 @@ mfe_status mfe_dot_f32(mfe_ctx* ctx, int64_t n, const float* x, const float* y,
  * (mfe_spmv, mfe_spmv_ell).  The context stays usable. */
 mfe_status mfe_inject_wait_timeout(mfe_ctx* ctx, int64_t wait_ns);
 
+/* The same for the solves whose iterations run in one resident kernel (small
+ * boxes, FP64 and mixed): at the first barrier of the next one on ctx its
+ * blocks wait for one arrival more than there are, give up after wait_ns
+ * nanoseconds (1 ms .. 2 s), and the solve returns MFE_TIMEOUT.  The context
+ * stays usable. */
+mfe_status mfe_inject_loop_fault(mfe_ctx* ctx, int64_t wait_ns);
+
 /* ------------------------------------------------------------------ */
 /* CG                                                                  */
 /* ------------------------------------------------------------------ */

@@ -32,8 +32,8 @@ __all__ = [
     "MiniFEError", "Context", "CSRMatrix", "CGResult", "default_context", "box_dims",
     "generate_matrix_structure", "assemble_FE_data", "impose_dirichlet", "box_bc_rows",
     "build_system", "matvec", "matvec_and_dot", "dot", "dot_f32", "waxpby", "fused_waxpby",
-    "inject_wait_timeout", "Stencil64", "matvec_stencil64", "set_multi_tuning", "cg_solve",
-    "cg_solve_host", "cg_solve_multi", "Batch", "batch_solve_boxes", "verify_solution",
+    "inject_wait_timeout", "inject_loop_fault", "Stencil64", "matvec_stencil64",
+    "set_multi_tuning", "cg_solve", "cg_solve_host", "cg_solve_multi", "Batch", "batch_solve_boxes", "verify_solution",
     "element_gradient", "to_f32", "spmm", "ELLMatrix", "matvec_ell", "cg_solve_ell",
 ]
 
@@ -475,6 +475,13 @@ def inject_wait_timeout(wait_ns: int = 20_000_000, ctx: Context | None = None):
     copies, so its bounded waits run out after wait_ns (mfe_inject_wait_timeout)."""
     ctx = ctx or default_context()
     ctx.check(ctx.lib.mfe_inject_wait_timeout(ctx.h, int(wait_ns)), "mfe_inject_wait_timeout")
+
+
+def inject_loop_fault(wait_ns: int = 20_000_000, ctx: Context | None = None):
+    """Test hook: the blocks of the context's next resident solver loop wait for one
+    that never arrives and give up after wait_ns (mfe_inject_loop_fault)."""
+    ctx = ctx or default_context()
+    ctx.check(ctx.lib.mfe_inject_loop_fault(ctx.h, int(wait_ns)), "mfe_inject_loop_fault")
 
 
 def fused_waxpby(alpha, x, beta, y, w, alpha2, x2, beta2, y2, w2, ctx: Context | None = None):

@@ -112,6 +112,7 @@ SIGNATURES = {
     "mfe_gather": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p]),
     "mfe_dot_f32": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_void_p, _P(c_double)]),
     "mfe_inject_wait_timeout": (ctypes.c_int, [c_void_p, c_int64]),
+    "mfe_inject_loop_fault": (ctypes.c_int, [c_void_p, c_int64]),
     "mfe_waxpby": (ctypes.c_int, [c_void_p, c_int64, c_double, c_void_p, c_double, c_void_p,
                                   c_void_p]),
     "mfe_fused_waxpby": (ctypes.c_int, [c_void_p, c_int64, c_double, c_void_p, c_double,

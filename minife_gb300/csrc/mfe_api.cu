@@ -588,6 +588,15 @@ mfe_status mfe_inject_wait_timeout(mfe_ctx* ctx, int64_t wait_ns)
   return MFE_OK;
 }
 
+mfe_status mfe_inject_loop_fault(mfe_ctx* ctx, int64_t wait_ns)
+{
+  if (!ctx) return MFE_BAD_ARG;
+  if (wait_ns < 1000000 || wait_ns > 2000000000)
+    return fail(ctx, MFE_BAD_ARG, "wait_ns must lie in [1 ms, 2 s]");
+  ctx->inject_loop_ns = (uint64_t)wait_ns;
+  return MFE_OK;
+}
+
 void mfe_cg_opts_default(mfe_cg_opts* o)
 {
   if (!o) return;

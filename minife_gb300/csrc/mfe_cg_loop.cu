@@ -51,7 +51,7 @@ struct LoopParams {
   int x_vec;               // x is 16-byte aligned
   CgState* st;
   double* partials;        // two sets of one per block: p.Ap, r.r
-  unsigned* arrived;       // blocks arrived at the barriers so far (0 at launch)
+  GridSync sync;
   int held;                // vectors that a block holds in shared memory (r, p, x, Ap in this order)
   int span;                // doubles of each
   int held_chunks;         // CSR operator: chunks of 32 rows whose values the block holds too
@@ -208,11 +208,11 @@ __device__ __forceinline__ void cg_loop(const LoopParams& P, double* held, Op&& 
       P.p[c0 + m - 1] = pv;
       if (P.held > 1) p1[m - 1] = pv;
     }
-    if (!(ok = grid_barrier(P.arrived, target += G))) break;
+    if (!(ok = grid_barrier(P.sync, target += G))) break;
     // Ap, p.Ap and the breakdown pre-test (cg_solve.hpp:179-198)
     const double dot = product(a1);
     ok = grid_sum<NT>(
-        dot, s_v, P.partials, P.arrived, target += G,
+        dot, s_v, P.partials, P.sync, target += G,
         [&](double total) {
           S.pAp = total;
           if (total < S.brkdown_tol) S.check_pending = 1;
@@ -234,9 +234,9 @@ __device__ __forceinline__ void cg_loop(const LoopParams& P, double* held, Op&& 
         pp = fma(pv, pv, pp);
         aa = fma(av, av, aa);
       }
-      ok = grid_sum<NT>(aa, s_v, P.partials + G, P.arrived, target += G, [&](double total) { s_alpha = total; });
+      ok = grid_sum<NT>(aa, s_v, P.partials + G, P.sync, target += G, [&](double total) { s_alpha = total; });
       if (!ok) break;
-      ok = grid_sum<NT>(pp, s_v, P.partials, P.arrived, target += G, [&](double total) {
+      ok = grid_sum<NT>(pp, s_v, P.partials, P.sync, target += G, [&](double total) {
         const double pAp = S.pAp;
         if (!(pAp < 0 || fabs(pAp) <= 100 * sqrt(s_alpha) * sqrt(total) * 2.220446049250313e-16)) {
           S.check_pending = 0;
@@ -284,7 +284,7 @@ __device__ __forceinline__ void cg_loop(const LoopParams& P, double* held, Op&& 
     }
     // the loop test of iteration k + 1 with the normr of the top of iteration
     // k (cg_solve.hpp:152-163)
-    ok = grid_sum<NT>(acc, s_v, P.partials + G, P.arrived, target += G, [&](double total) {
+    ok = grid_sum<NT>(acc, s_v, P.partials + G, P.sync, target += G, [&](double total) {
       S.rr_new = total;
       S.num_iters = S.k;
       S.p_reset = 0;
@@ -317,7 +317,7 @@ __device__ __forceinline__ void cg_loop(const LoopParams& P, double* held, Op&& 
     if (tid == 0) atomicOr(&P.st->err, ERR_WAIT_TIMEOUT);
   } else if (blockIdx.x == 0 && tid == 0) {
     if (S.check_pending) S.normr = s_normr;
-    *P.st = S;
+    store_state(P.st, S);
   }
 }
 
@@ -479,8 +479,7 @@ mfe_status launch_cg_loop(mfe_ctx* ctx, const mfe_csr* A, const CgLoopArgs& a)
   double* ws = static_cast<double*>(workspace(ctx, "cg.loop", sizeof(double) * 4096 + 16));
   if (!ws) return fail(ctx, MFE_OOM, "CG workspace allocation failed");
   P.partials = ws;
-  P.arrived = reinterpret_cast<unsigned*>(ws + 4096);
-  MFE_CUDA_TRY(ctx, cudaMemsetAsync(P.arrived, 0, sizeof(unsigned), ctx->stream));
+  MFE_TRY(start_sync(ctx, reinterpret_cast<unsigned*>(ws + 4096), &P.sync));
   // 256 threads while they leave room for most values, else 384, us per
   // iteration: 48 x 40 x 56 17.2 / 16.9, 56^3 22.2 / 24.0, 64^3 31.1 / 28.8,
   // 80^3 48.5 / 45.3 (512: 50.2).

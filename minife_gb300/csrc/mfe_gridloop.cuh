@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <mutex>
 
 #include "mfe_common.cuh"
@@ -11,29 +12,36 @@
 
 namespace mfe {
 
+// What the blocks of a loop meet by: how many have arrived at its barriers so far,
+// and how long one waits for the others.
+struct GridSync {
+  unsigned* arrived;
+  uint64_t wait_ns;
+};
+
 // The calling thread's block arrives at a barrier of all blocks and waits;
 // false after the time limit.
-__device__ __forceinline__ bool arrive_and_wait(unsigned* arrived, unsigned target)
+__device__ __forceinline__ bool arrive_and_wait(const GridSync& sync, unsigned target)
 {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sync.arrived) : "memory");
   auto there = [&] {
     unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(sync.arrived) : "memory");
     return (int)(v - target) >= 0;
   };
   if (there()) return true;
   const uint64_t t0 = global_ns();
   for (unsigned i = 1; !there(); ++i)
-    if ((i & 255u) == 0 && global_ns() - t0 > kWaitLimitNs) return false;
+    if ((i & 255u) == 0 && global_ns() - t0 > sync.wait_ns) return false;
   return true;
 }
 
 // All blocks; false (in every thread of the block) after the time limit.
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target)
+__device__ __forceinline__ bool grid_barrier(const GridSync& sync, unsigned target)
 {
   __shared__ bool s_ok;
   __syncthreads();
-  if (threadIdx.x == 0) s_ok = arrive_and_wait(arrived, target);
+  if (threadIdx.x == 0) s_ok = arrive_and_wait(sync, target);
   __syncthreads();
   return s_ok;
 }
@@ -45,7 +53,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target)
 // after the grid barrier the blocks' sums in block order.  s_v: a double per
 // thread; beside(): what thread 32 does meanwhile.
 template <int NT, typename Then, typename Beside>
-__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, unsigned* arrived, unsigned target,
+__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, const GridSync& sync, unsigned target,
                                          Then&& then, Beside&& beside)
 {
   __shared__ bool s_ok;
@@ -59,7 +67,7 @@ __device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, u
     bool ok = true;
     if (threadIdx.x == 0) {
       __stcg(slots + blockIdx.x, bt);
-      ok = arrive_and_wait(arrived, target);
+      ok = arrive_and_wait(sync, target);
     }
     __syncwarp();
     double t[4] = {0.0, 0.0, 0.0, 0.0};
@@ -77,10 +85,10 @@ __device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, u
 }
 
 template <int NT, typename Then>
-__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, unsigned* arrived, unsigned target,
+__device__ __forceinline__ bool grid_sum(double v, double* s_v, double* slots, const GridSync& sync, unsigned target,
                                          Then&& then)
 {
-  return grid_sum<NT>(v, s_v, slots, arrived, target, then, [] {});
+  return grid_sum<NT>(v, s_v, slots, sync, target, then, [] {});
 }
 
 // A block's share of the vectors: a range that begins at a multiple of A (a
@@ -89,6 +97,18 @@ template <int A>
 __device__ __forceinline__ int64_t share(int64_t n, unsigned b, unsigned nb)
 {
   return b == nb ? n : (n * b / nb) & ~(int64_t)(A - 1);
+}
+
+// A loop's state back to memory, but for its error word: another block may have set
+// that after its last wait.
+template <typename State>
+__device__ __forceinline__ void store_state(State* to, const State& from)
+{
+  static_assert(sizeof(State) % sizeof(unsigned) == 0, "words");
+  const unsigned* f = reinterpret_cast<const unsigned*>(&from);
+  unsigned* t = reinterpret_cast<unsigned*>(to);
+  for (size_t i = 0; i < sizeof(State) / sizeof(unsigned); ++i)
+    if (i != offsetof(State, err) / sizeof(unsigned)) t[i] = f[i];
 }
 
 // Shared memory for a block's static part and the system's, out of 227 KB per
@@ -102,6 +122,18 @@ inline size_t plan_held(int64_t n, int g, size_t elem, size_t room, int most, in
   *span = (int)((ceil_div(n, (int64_t)g) + 7) & ~(int64_t)3);
   *held = (int)std::min<size_t>(room / (elem * *span), most);
   return elem * *span * *held;
+}
+
+// The loop's count of arrivals set to zero on the stream.  A pending
+// mfe_inject_loop_fault sets it one short instead, so that no block ever sees all
+// of them arrive and each gives up after the injected time.
+inline mfe_status start_sync(mfe_ctx* ctx, unsigned* arrived, GridSync* sync)
+{
+  sync->arrived = arrived;
+  sync->wait_ns = ctx->inject_loop_ns ? ctx->inject_loop_ns : kWaitLimitNs;
+  MFE_CUDA_TRY(ctx, cudaMemsetAsync(arrived, ctx->inject_loop_ns ? 0xff : 0, sizeof(unsigned), ctx->stream));
+  ctx->inject_loop_ns = 0;
+  return MFE_OK;
 }
 
 // A loop's blocks fill the device and wait for one another, so two of them must

@@ -36,6 +36,9 @@ struct mfe_ctx {
   // kernel, the warp-staged CSR and ELL kernels) launched outside a graph
   // capture withholds its copies; its waits give up after this long
   uint64_t inject_wait_ns = 0;
+  // mfe_inject_loop_fault: the blocks of the next resident loop wait this long for
+  // one that never arrives (0: none pending)
+  uint64_t inject_loop_ns = 0;
   // launch shape of the multi-RHS stencil SpMM (mfe_multi_set_tuning): z
   // steps per work item, 0 = the default
   int multi_zchunk = 0;

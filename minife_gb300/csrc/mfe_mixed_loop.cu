@@ -33,7 +33,7 @@ struct MixLoopParams {
   float* Ap;
   MixState* st;
   double* partials;   // two sets of one per block: p.Ap, r.r
-  unsigned* arrived;
+  GridSync sync;
   int held, span;     // vectors held (r, p, x, Ap in this order), floats of each
   int Nx, Ny, Nz, Nxp, NP;
   float w[8], dd;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(NT, 1) k_mx_loop(const __grid_constant__ MixLo
       pg[i] = pv;
       if (P.held > 1) p4[i] = pv;
     }
-    if (!(ok = grid_barrier(P.arrived, target += G))) break;
+    if (!(ok = grid_barrier(P.sync, target += G))) break;
     DFAcc dot;
     for (int f = 30 * warp; f < m; f += 30 * (NT / 32)) {
       const int i = f + lane - 1;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(NT, 1) k_mx_loop(const __grid_constant__ MixLo
         dot.add_product(y, pr);
       }
     }
-    ok = grid_sum<NT>(dot.value(), s_v, P.partials, P.arrived, target += G, [&](double total) {
+    ok = grid_sum<NT>(dot.value(), s_v, P.partials, P.sync, target += G, [&](double total) {
       S.pAp = total;
       s_alpha = total > 0.0 ? (float)(S.rr / total) : 0.0f;
     });
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(NT, 1) k_mx_loop(const __grid_constant__ MixLo
       acc.add_product(rv.z, rv.z);
       acc.add_product(rv.w, rv.w);
     }
-    ok = grid_sum<NT>(acc.value(), s_v, P.partials + G, P.arrived, target += G, [&](double total) {
+    ok = grid_sum<NT>(acc.value(), s_v, P.partials + G, P.sync, target += G, [&](double total) {
       S.rr_new = total;
       S.alpha_prev = alpha;
       S.x_pending = 1;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(NT, 1) k_mx_loop(const __grid_constant__ MixLo
   if (!ok) {
     if (tid == 0) atomicOr(&P.st->err, ERR_WAIT_TIMEOUT);
   } else if (blockIdx.x == 0 && tid == 0) {
-    *P.st = S;
+    store_state(P.st, S);
   }
 }
 
@@ -217,8 +217,7 @@ mfe_status launch_mixed_loop(mfe_ctx* ctx, const mfe_csr* A, const float* coef, 
   double* ws = static_cast<double*>(workspace(ctx, "mixed.loop", sizeof(double) * 4096 + 16));
   if (!ws) return fail(ctx, MFE_OOM, "mixed solver workspace allocation failed");
   P.partials = ws;
-  P.arrived = reinterpret_cast<unsigned*>(ws + 4096);
-  MFE_CUDA_TRY(ctx, cudaMemsetAsync(P.arrived, 0, sizeof(unsigned), ctx->stream));
+  MFE_TRY(start_sync(ctx, reinterpret_cast<unsigned*>(ws + 4096), &P.sync));
   // 512 threads against 1024, us per iteration: 64^3 14.0 / 14.9, 97 x 64 x 130
   // 18.5 / 18.6, 110^3 24.5 / 23.3, 124^3 30.1 / 27.7
   return P.n <= 6000 * (int64_t)ctx->sm_count ? run_mx_loop<512>(ctx, P) : run_mx_loop<1024>(ctx, P);
