@@ -252,7 +252,8 @@ mfe_status mfe_inject_wait_timeout(mfe_ctx* ctx, int64_t wait_ns);
  * boxes, FP64 and mixed): at the first barrier of the next one on ctx its
  * blocks wait for one arrival more than there are, give up after wait_ns
  * nanoseconds (1 ms .. 2 s), and the solve returns MFE_TIMEOUT.  The context
- * stays usable. */
+ * stays usable.  wait_ns 0: the next one is refused, as by a device that cannot
+ * hold all its blocks, and the solve runs as a graph. */
 mfe_status mfe_inject_loop_fault(mfe_ctx* ctx, int64_t wait_ns);
 
 /* ------------------------------------------------------------------ */

@@ -479,7 +479,8 @@ def inject_wait_timeout(wait_ns: int = 20_000_000, ctx: Context | None = None):
 
 def inject_loop_fault(wait_ns: int = 20_000_000, ctx: Context | None = None):
     """Test hook: the blocks of the context's next resident solver loop wait for one
-    that never arrives and give up after wait_ns (mfe_inject_loop_fault)."""
+    that never arrives and give up after wait_ns; 0: it is refused, and the solve runs
+    as a graph (mfe_inject_loop_fault)."""
     ctx = ctx or default_context()
     ctx.check(ctx.lib.mfe_inject_loop_fault(ctx.h, int(wait_ns)), "mfe_inject_loop_fault")
 

@@ -591,9 +591,9 @@ mfe_status mfe_inject_wait_timeout(mfe_ctx* ctx, int64_t wait_ns)
 mfe_status mfe_inject_loop_fault(mfe_ctx* ctx, int64_t wait_ns)
 {
   if (!ctx) return MFE_BAD_ARG;
-  if (wait_ns < 1000000 || wait_ns > 2000000000)
-    return fail(ctx, MFE_BAD_ARG, "wait_ns must lie in [1 ms, 2 s]");
-  ctx->inject_loop_ns = (uint64_t)wait_ns;
+  if (wait_ns != 0 && (wait_ns < 1000000 || wait_ns > 2000000000))
+    return fail(ctx, MFE_BAD_ARG, "wait_ns must be 0 or lie in [1 ms, 2 s]");
+  ctx->inject_loop_ns = wait_ns;
   return MFE_OK;
 }
 

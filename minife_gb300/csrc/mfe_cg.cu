@@ -594,7 +594,7 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
   // (mfe_cg_loop.cu).  Where the lines lie, us per iteration, graph against
   // loop: CSR values 96^3 81.8 / 80.7 and 112^3 112.8 / 116.3; stencil
   // operator 112^3 57.4 / 51.4, 128^3 73.1 / 72.5 and 144^3 90.9 / 94.1.
-  const bool loop = !eager && getenv("MFE_SPMV_GENERIC") == nullptr && !sell && csr_is_box(&A) &&
+  bool loop = !eager && getenv("MFE_SPMV_GENERIC") == nullptr && !sell && csr_is_box(&A) &&
                     A.dtype == MFE_F64 && n <= (B.st64 ? 2000000 : 1000000);
   // (re)build the graph when the operands changed
   const void* key[12] = {A.row_offsets, A.cols, A.vals, x, b, B.r, B.p, B.Ap, B.st,
@@ -605,10 +605,12 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
   double op[10] = {B.st64 ? 1.0 : 0.0, B.dd};
   for (int c = 0; c < 8; ++c) op[2 + c] = B.w8[c];
   mfe_cg_graph* g = ctx->cg_graph;
-  if (!eager && !loop &&
-      (!g || g->n != n || g->stream != ctx->stream || memcmp(g->key, key, sizeof(key)) != 0 ||
-       memcmp(g->op, op, sizeof(op)) != 0)) {
+  auto ready_graph = [&]() -> mfe_status {
+    if (g && g->n == n && g->stream == ctx->stream && memcmp(g->key, key, sizeof(key)) == 0 &&
+        memcmp(g->op, op, sizeof(op)) == 0)
+      return MFE_OK;
     cg_graph_destroy(g);
+    g = nullptr;
     ctx->cg_graph = nullptr;
     MFE_TRY(build_graph(ctx, &A, x, B, rb, &g));
     memcpy(g->key, key, sizeof(key));
@@ -616,7 +618,9 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
     g->n = n;
     g->stream = ctx->stream;
     ctx->cg_graph = g;
-  }
+    return MFE_OK;
+  };
+  if (!eager && !loop) MFE_TRY(ready_graph());
 
   int status = MFE_OK;
   bool confirmed = spec == nullptr;
@@ -634,10 +638,14 @@ static mfe_status cg_f64(mfe_ctx* ctx, const mfe_csr* A_in, const double* b, dou
         }
       } else if (loop) {
         const CgLoopArgs args{x, B.r, B.p, B.Ap, B.st, B.st64 ? B.w8 : nullptr, B.dd};
-        MFE_TRY(launch_cg_loop(ctx, &A, args));
-      } else {
-        MFE_CUDA_TRY(ctx, cudaGraphLaunch(g->exec, ctx->stream));
+        const mfe_status st = launch_cg_loop(ctx, &A, args);
+        if (st != MFE_OK && st != MFE_NOT_SUPPORTED) return st;
+        if (st == MFE_NOT_SUPPORTED) {  // not on this device: the graph from here on
+          loop = false;
+          MFE_TRY(ready_graph());
+        }
       }
+      if (!eager && !loop) MFE_CUDA_TRY(ctx, cudaGraphLaunch(g->exec, ctx->stream));
       MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, B.st, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
       MFE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
       if (hs->err) return fail(ctx, MFE_TIMEOUT, "a bounded device wait gave up during CG");

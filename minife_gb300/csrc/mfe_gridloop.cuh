@@ -129,10 +129,11 @@ inline size_t plan_held(int64_t n, int g, size_t elem, size_t room, int most, in
 // of them arrive and each gives up after the injected time.
 inline mfe_status start_sync(mfe_ctx* ctx, unsigned* arrived, GridSync* sync)
 {
+  const bool fault = ctx->inject_loop_ns > 0;
   sync->arrived = arrived;
-  sync->wait_ns = ctx->inject_loop_ns ? ctx->inject_loop_ns : kWaitLimitNs;
-  MFE_CUDA_TRY(ctx, cudaMemsetAsync(arrived, ctx->inject_loop_ns ? 0xff : 0, sizeof(unsigned), ctx->stream));
-  ctx->inject_loop_ns = 0;
+  sync->wait_ns = fault ? (uint64_t)ctx->inject_loop_ns : kWaitLimitNs;
+  MFE_CUDA_TRY(ctx, cudaMemsetAsync(arrived, fault ? 0xff : 0, sizeof(unsigned), ctx->stream));
+  if (fault) ctx->inject_loop_ns = -1;
   return MFE_OK;
 }
 
@@ -150,11 +151,17 @@ inline LoopOrder& loop_order(int device)
 }
 
 // The attribute set and the occupancy asked for, once per kernel and device; a
-// launch of blocks that would not all be resident is refused.
+// launch of blocks that would not all be resident is refused (MFE_NOT_SUPPORTED:
+// fewer blocks fit an SM, or fewer SMs are there for this process than the device
+// has).
 template <size_t kMost>
 inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads, int per_sm, size_t smem,
                        std::atomic<int>* ready, void** args)
 {
+  if (ctx->inject_loop_ns == 0) {
+    ctx->inject_loop_ns = -1;
+    return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel was refused (injected)");
+  }
   std::atomic<int>& have = ready[ctx->device & 63];
   if (have.load(std::memory_order_acquire) == 0) {
     int blocks = 0;
@@ -167,7 +174,12 @@ inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads
   std::lock_guard<std::mutex> lock(order.mu);
   if (!order.last) MFE_CUDA_TRY(ctx, cudaEventCreateWithFlags(&order.last, cudaEventDisableTiming));
   MFE_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, order.last, 0));
-  MFE_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream));
+  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
+  }
+  MFE_CUDA_TRY(ctx, e);
   MFE_CUDA_TRY(ctx, cudaEventRecord(order.last, ctx->stream));
   return MFE_OK;
 }

@@ -37,8 +37,8 @@ struct mfe_ctx {
   // capture withholds its copies; its waits give up after this long
   uint64_t inject_wait_ns = 0;
   // mfe_inject_loop_fault: the blocks of the next resident loop wait this long for
-  // one that never arrives (0: none pending)
-  uint64_t inject_loop_ns = 0;
+  // one that never arrives, or (0) the loop is refused (-1: none pending)
+  int64_t inject_loop_ns = -1;
   // launch shape of the multi-RHS stencil SpMM (mfe_multi_set_tuning): z
   // steps per work item, 0 = the default
   int multi_zchunk = 0;
@@ -221,12 +221,13 @@ struct CgLoopArgs {
   const double* w8;
   double dd;
 };
+// MFE_NOT_SUPPORTED, with nothing launched, when the device cannot hold its blocks.
 mfe_status launch_cg_loop(mfe_ctx* ctx, const mfe_csr* A, const CgLoopArgs& a);
 
 // ---- mixed-precision CG in one cooperative kernel (mfe_mixed_loop.cu) ----
 // FP32 iterations with the mirror-symmetric stencil coef until a reliable update
 // is due or the solve ends; st is the MixState, p has stencil_ghost zero rows
-// on both sides, the vectors are x-padded.
+// on both sides, the vectors are x-padded.  MFE_NOT_SUPPORTED as launch_cg_loop.
 mfe_status launch_mixed_loop(mfe_ctx* ctx, const mfe_csr* A, const float* coef, float* r, float* p, float* x32,
                              float* Ap, void* st);
 

@@ -414,17 +414,24 @@ mfe_status cg_mixed(mfe_ctx* ctx, const mfe_csr* A64_in, const double* b, double
   grid_for(ctx, 1, (const void*)k_mx_xupdate);
   const bool eager = getenv("MFE_CG_EAGER") != nullptr;
   float w8[8];
-  const bool loop = !eager && B.stencil && n <= kLoopRows && stencil_mirror_classes(B.coef, w8);
+  bool loop = !eager && B.stencil && n <= kLoopRows && stencil_mirror_classes(B.coef, w8);
   if (eager || loop) {
     for (;;) {
       MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, B.st, sizeof(MixState), cudaMemcpyDeviceToHost, ctx->stream));
       MFE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
       if (!hs->cont || hs->err) break;
-      if (loop) MFE_TRY(launch_mixed_loop(ctx, &A64, B.coef, B.r, B.p, B.x32, B.Ap, B.st));
-      else MFE_TRY(launch_iter(ctx, A32, A64, b, x, B, 0, 0, 0));
+      if (loop) {
+        const mfe_status st = launch_mixed_loop(ctx, &A64, B.coef, B.r, B.p, B.x32, B.Ap, B.st);
+        if (st != MFE_OK && st != MFE_NOT_SUPPORTED) return st;
+        loop = st == MFE_OK;
+        if (!loop) break;  // not on this device: the graph from here on
+      } else {
+        MFE_TRY(launch_iter(ctx, A32, A64, b, x, B, 0, 0, 0));
+      }
       MFE_TRY(launch_update(ctx, A64, b, x, B, 0, 0));
     }
-  } else {
+  }
+  if (!eager && !loop) {
     GraphLoop L;
     L.begin = [&](cudaGraphConditionalHandle h) {
       k_mx_begin<<<1, 1, 0, ctx->stream>>>(B.st, h);
