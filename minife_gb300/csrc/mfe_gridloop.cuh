@@ -170,16 +170,25 @@ inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads
     if (blocks < per_sm) return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
     have.store(blocks, std::memory_order_release);
   }
+  auto launch = [&]() -> mfe_status {
+    const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
+    }
+    MFE_CUDA_TRY(ctx, e);
+    return MFE_OK;
+  };
+  // a capture launches nothing (the solve's first read of its state ends it), and an
+  // event recorded in one could not be waited for any more
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  MFE_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return launch();
   LoopOrder& order = loop_order(ctx->device);
   std::lock_guard<std::mutex> lock(order.mu);
   if (!order.last) MFE_CUDA_TRY(ctx, cudaEventCreateWithFlags(&order.last, cudaEventDisableTiming));
   MFE_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, order.last, 0));
-  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    cudaGetLastError();
-    return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
-  }
-  MFE_CUDA_TRY(ctx, e);
+  MFE_TRY(launch());
   MFE_CUDA_TRY(ctx, cudaEventRecord(order.last, ctx->stream));
   return MFE_OK;
 }
