@@ -416,11 +416,16 @@ __global__ void __launch_bounds__(NT, NB)
   });
 }
 
+// Half of the SMs while they take 128 rows each: 76 blocks against 152, us per
+// iteration, CSR values / stencil, 18^3 10.5, 11.6 / 11.5, 12.6; 21^3 10.6, 11.2 / 10.9,
+// 11.7; 24^3 11.4, 12.4 / 10.8, 11.6.
+int fp64_blocks(const mfe_ctx* ctx, int64_t n) { return loop_blocks(ctx, n, 64, 64 * (int64_t)ctx->sm_count); }
+
 template <int NT>
 mfe_status run_stencil(mfe_ctx* ctx, LoopParams& P)
 {
   static std::atomic<int> ready[64];
-  const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(P.n, 64), ctx->sm_count));
+  const int g = fp64_blocks(ctx, P.n);
   const size_t smem = plan_held(P.n, g, sizeof(double), kRoom, 4, &P.span, &P.held);
   void* args[] = {&P};
   return coop_launch<kRoom>(ctx, (const void*)k_cg_loop_stencil<NT>, g, NT, 1, smem, ready, args);
@@ -431,7 +436,7 @@ mfe_status run_csr(mfe_ctx* ctx, LoopParams& P)
 {
   static std::atomic<int> ready[64];
   constexpr size_t kChunkBytes = kChunk * sizeof(double), kBuffers = NT / 32 * kChunkBytes;
-  const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(P.n, 64), ctx->sm_count));
+  const int g = fp64_blocks(ctx, P.n);
   // all values beside all vectors, or the buffers, then vectors, then values
   size_t smem = plan_held(P.n, g, sizeof(double), kRoom, 4, &P.span, &P.held);
   const int chunks = (P.span + 31) / 32;

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstddef>
 #include <mutex>
+#include <vector>
 
 #include "mfe_common.cuh"
 #include "mfe_internal.h"
@@ -115,6 +116,14 @@ __device__ __forceinline__ void store_state(State* to, const State& from)
 // block and 228 KB per SM.
 constexpr size_t kReserved = 8 * 1024, kRoom = 227 * 1024 - kReserved;
 
+// Blocks of at least `rows` entries, one per SM, on half of the SMs up to `half`
+// entries: there the shares cost nothing, and two loops run side by side.
+inline int loop_blocks(const mfe_ctx* ctx, int64_t n, int rows, int64_t half)
+{
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, (int64_t)rows),
+                                                     n <= half ? (ctx->sm_count + 1) / 2 : ctx->sm_count));
+}
+
 // How many of its vectors (n elements of elem bytes over g blocks) a block can
 // hold in `room` bytes, at most `most`; the bytes they take.
 inline size_t plan_held(int64_t n, int g, size_t elem, size_t room, int most, int* span, int* held)
@@ -137,17 +146,83 @@ inline mfe_status start_sync(mfe_ctx* ctx, unsigned* arrived, GridSync* sync)
   return MFE_OK;
 }
 
-// A loop's blocks fill the device and wait for one another, so two of them must
-// never hold parts of it: each launch, of any context and stream, waits on the
-// device for the one before it.
+// A loop's blocks wait for one another, so two loops must never each hold a part
+// of the device that the other needs.  A block may fill an SM, so loops (of any
+// context and stream) run side by side while they have no more blocks together than
+// the device has SMs: then a block that has not started always finds an SM without
+// any.  A launch waits on the device for the oldest of the running ones until that
+// holds.  (Whatever else runs on an SM ends by itself.)
+// Measured, us per solve with 1, 2, 4 and 8 threads solving (1e-9): FP64 stencil 8^3
+// 340, 180, 92, 74 (one loop after another 345, 181, 176, 171; as graphs 610, 333,
+// 181, 156); 16^3 519, 292, 225, 189 (515, 373, 374, 371; 1040, 563, 295, 263); mixed
+// 24^3 939, 505, 392, 366 (982, 736, 690, 677; 1451, 1369, 1080, 910).  Loops that fill
+// the device go one after another: 30^3 916, 848, 784, 772, where graphs take 2303,
+// 1154, 621, 555 (with more than two threads the graphs' gaps fill up); 64^3 3641,
+// 3579, 3513, 3533 (7519, 5110, 4011, 3990).
 struct LoopOrder {
+  struct Loop {
+    cudaEvent_t end;
+    int blocks;
+  };
   std::mutex mu;
-  cudaEvent_t last = nullptr;
+  std::vector<Loop> running;  // in the order of their launches
+  std::vector<cudaEvent_t> spare;
 };
 inline LoopOrder& loop_order(int device)
 {
   static LoopOrder order[64];
   return order[device & 63];
+}
+
+// launch() on ctx->stream beside the loops that run, as blocks allow
+template <typename Launch>
+mfe_status launch_in_order(mfe_ctx* ctx, int blocks, Launch&& launch)
+{
+  // a capture launches nothing (and the solve's first read of its state ends it)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  MFE_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return launch();
+  blocks = std::min(blocks, ctx->sm_count);
+  LoopOrder& order = loop_order(ctx->device);
+  std::lock_guard<std::mutex> lock(order.mu);
+  // (asking for an event must not end a capture that another thread has begun)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  MFE_CUDA_TRY(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+  int held = 0;
+  for (size_t i = 0; i < order.running.size();) {
+    if (cudaEventQuery(order.running[i].end) == cudaSuccess) {
+      order.spare.push_back(order.running[i].end);
+      order.running.erase(order.running.begin() + i);
+    } else {
+      held += order.running[i++].blocks;
+    }
+  }
+  cudaGetLastError();  // (cudaErrorNotReady)
+  cudaError_t e = cudaSuccess;
+  cudaEvent_t end = nullptr;
+  if (order.spare.empty()) {
+    e = cudaEventCreateWithFlags(&end, cudaEventDisableTiming);
+  } else {
+    end = order.spare.back();
+    order.spare.pop_back();
+  }
+  const cudaError_t e2 = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e == cudaSuccess) e = e2;
+  for (size_t i = 0; e == cudaSuccess && i < order.running.size() && held + blocks > ctx->sm_count; ++i) {
+    e = cudaStreamWaitEvent(ctx->stream, order.running[i].end, 0);
+    held -= order.running[i].blocks;
+  }
+  mfe_status st = e == cudaSuccess ? launch() : cuda_fail(ctx, e, "the order of the solvers' loops");
+  if (st == MFE_OK) {
+    e = cudaEventRecord(end, ctx->stream);
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(ctx->stream);  // nothing may start beside it unseen
+      st = cuda_fail(ctx, e, "the order of the solvers' loops");
+    }
+  }
+  if (st == MFE_OK) order.running.push_back({end, blocks});
+  else if (end) order.spare.push_back(end);
+  return st;
 }
 
 // The attribute set and the occupancy asked for, once per kernel and device; a
@@ -170,7 +245,7 @@ inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads
     if (blocks < per_sm) return fail(ctx, MFE_NOT_SUPPORTED, "a solver's loop kernel does not fit the device");
     have.store(blocks, std::memory_order_release);
   }
-  auto launch = [&]() -> mfe_status {
+  return launch_in_order(ctx, g, [&]() -> mfe_status {
     const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(g), dim3(threads), args, smem, ctx->stream);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
@@ -178,19 +253,7 @@ inline mfe_status coop_launch(mfe_ctx* ctx, const void* kern, int g, int threads
     }
     MFE_CUDA_TRY(ctx, e);
     return MFE_OK;
-  };
-  // a capture launches nothing (the solve's first read of its state ends it), and an
-  // event recorded in one could not be waited for any more
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  MFE_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return launch();
-  LoopOrder& order = loop_order(ctx->device);
-  std::lock_guard<std::mutex> lock(order.mu);
-  if (!order.last) MFE_CUDA_TRY(ctx, cudaEventCreateWithFlags(&order.last, cudaEventDisableTiming));
-  MFE_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, order.last, 0));
-  MFE_TRY(launch());
-  MFE_CUDA_TRY(ctx, cudaEventRecord(order.last, ctx->stream));
-  return MFE_OK;
+  });
 }
 
 }  // namespace mfe
