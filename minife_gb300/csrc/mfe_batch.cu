@@ -1591,7 +1591,7 @@ BxList bx_list(int* base, int nbox, int which)
 // Runs `body` as a CUDA graph with a conditional while node on ctl->cont (or,
 // with MFE_CG_EAGER set, as a host loop reading cont back each iteration).
 template <typename Body>
-mfe_status bx_loop(mfe_ctx* ctx, BatchCtl* dctl, Body body)
+mfe_status bx_loop(mfe_ctx* ctx, BatchCtl* dctl, int copies, Body body)
 {
   if (getenv("MFE_CG_EAGER") != nullptr) {
     BatchCtl* hctl = static_cast<BatchCtl*>(host_scratch(ctx, sizeof(BatchCtl)));
@@ -1612,7 +1612,7 @@ mfe_status bx_loop(mfe_ctx* ctx, BatchCtl* dctl, Body body)
   // The kernels of a reliable update run empty where no box takes one: a
   // conditional node per iteration for them measured 35.8 ms against 34.9
   // (24 boxes of 16..96 to 1e-13), one iteration per test 36.0.
-  L.copies = 4;
+  L.copies = copies;
   return run_graph_loop(ctx, L, "batched CG graph");
 }
 
@@ -1849,7 +1849,14 @@ mfe_status batch_solve(mfe_ctx* ctx, mfe_batch* bt, const mfe_cg_opts* o, double
                         (const void*)k_bx_xupdate, (const void*)k_bx_p<double>,
                         (const void*)k_bx_update<double>})
     bx_vgrid(ctx, k);
-  MFE_TRY(bx_loop(ctx, bt->ctl, [&](cudaGraphConditionalHandle h, int in_graph) -> mfe_status {
+  // four iterations a body, where no single update ends it (every box has its own);
+  // whole solves, one / four: four boxes of 3^3 elements, of 1, 3 and 10 iterations 224,
+  // 280, 497 / 314, 345, 555 us; eight of 48^3, of 10 and 30 884, 1694 / 898, 1668
+  mfe_cg_opts all = *o;
+  all.refine_k = INT_MAX;
+  all.inner_tol = 0.0;
+  const int side = *std::max_element(bt->dims.begin(), bt->dims.end());
+  MFE_TRY(bx_loop(ctx, bt->ctl, loop_copies(&all, side, 4, 24), [&](cudaGraphConditionalHandle h, int in_graph) -> mfe_status {
     return R.mixed ? bx_iter_mixed(ctx, R, h, in_graph) : bx_iter_f64(ctx, R, h, in_graph);
   }));
   MFE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, ctx->stream));

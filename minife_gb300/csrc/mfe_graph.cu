@@ -1,4 +1,6 @@
 // The solvers' device-side loops: one CUDA graph with a conditional while node.
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "mfe_internal.h"
@@ -52,6 +54,20 @@ cudaError_t capture(cudaStream_t s, cudaGraph_t g, Deps& deps, mfe_status* st, F
 }
 
 }  // namespace
+
+// The iterations that CG takes for a digit of the residual: about a quarter of the
+// box's longest side.
+int loop_copies(const mfe_cg_opts* o, int side, int most, int worth)
+{
+  const double digits = o->tol_mode == MFE_TOL_RELATIVE ? -std::log10(std::max(o->tol, 1e-17)) : 16.0;
+  const double iterations = std::min<double>(o->max_iter, 0.25 * side * std::max(digits, 0.0));
+  if (iterations < worth) return 1;
+  const double per_update = 1.0 + 0.25 * side * -0.5 * std::log10(mixed_delta2(o));
+  const double between = o->refine_k > 0 ? std::min<double>(o->refine_k, per_update) : per_update;
+  int copies = most;
+  while (copies > 1 && copies > between) copies /= 2;
+  return copies;
+}
 
 mfe_status run_graph_loop(mfe_ctx* ctx, const GraphLoop& L, const char* where)
 {

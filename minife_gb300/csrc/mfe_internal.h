@@ -87,6 +87,12 @@ struct GraphLoop {
   int copies = 1;
 };
 mfe_status run_graph_loop(mfe_ctx* ctx, const GraphLoop& L, const char* where);
+// How many iterations the body should hold, at most `most` (a power of two): no more
+// than lie between two updates (each ends the body early, and the rest of its
+// kernels run empty), and one when the solve is expected to end before `worth`
+// iterations, as each copy is captured and instantiated on every call.  side: the
+// elements of the longest side of the (largest) box.
+int loop_copies(const mfe_cg_opts* o, int side, int most, int worth);
 
 // ---- assembly (mfe_assemble.cu) ----
 mfe_status launch_structure(mfe_ctx* ctx, int nx, int ny, int nz, int32_t* ro, int32_t* cols);

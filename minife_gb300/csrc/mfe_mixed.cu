@@ -44,6 +44,9 @@ constexpr int kMaxPart = 8192;
 // iterations in a row in the loop's body (160 x 192 x 144, us per iteration: 1
 // 46.5, 2 43.5, 4 41.6, 8 40.9; 40^3: 22.7, 19.7, 18.1, 17.6)
 constexpr int kCopies = 8;
+// (160^3, whole solves of 1, 3, 10 and 30 iterations: one copy 1154, 1225, 1483, 2487
+// us, eight 1193, 1254, 1501, 2466)
+constexpr int kCopiesWorth = 16;
 // up to here the iterations between two reliable updates run in one kernel
 // (mfe_mixed_loop.cu: 124^3 27.7 us per iteration against 29.1 here, 160 x 192 x
 // 144 50 against 40.5)
@@ -443,7 +446,8 @@ mfe_status cg_mixed(mfe_ctx* ctx, const mfe_csr* A64_in, const double* b, double
       return launch_iter(ctx, A32, A64, b, x, B, h, hu, 1);
     };
     L.update = [&](cudaGraphConditionalHandle h) { return launch_update(ctx, A64, b, x, B, h, 1); };
-    L.copies = B.stencil ? kCopies : 1;
+    const int side = std::max({A64.box_nx, A64.box_ny, A64.box_nz});
+    L.copies = B.stencil ? loop_copies(o, side, kCopies, kCopiesWorth) : 1;
     MFE_TRY(run_graph_loop(ctx, L, "mixed CG graph"));
   }
   MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, B.st, sizeof(MixState), cudaMemcpyDeviceToHost, ctx->stream));

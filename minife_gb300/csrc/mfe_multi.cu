@@ -44,6 +44,10 @@ constexpr int kMaxPartM = 2048;
 constexpr int kGroupM = 32;
 constexpr int kPartsM = kMaxPartM + kMaxPartM / kGroupM;
 constexpr int kTicketsM = 1 + kMaxPartM / kGroupM;
+// iterations in the loop's body with the stencil, and how many a solve must take to
+// repay them (whole solves of 1, 10, 20 and 30 iterations, one copy / eight: 8^3 x 32 306,
+// 542, 845 / 415, 622, 905 us; 32^3 x 32 419, 743, 1087, 1527 / 483, 758, 1070, 1505)
+constexpr int kCopiesM = 8, kCopiesWorthM = 24;
 
 // stage capacities (elements): a tile's values, and one x segment of
 // kTileRowsM + 2 rows of nrhs values, each with room for rounding both ends
@@ -1655,7 +1659,7 @@ mfe_status cg_multi(mfe_ctx* ctx, const mfe_csr* A64_in, int nrhs, const double*
         [&](cudaGraphConditionalHandle h, int in_graph) {
           return multi_update_mixed(ctx, A64, nrhs, B, X, W, h, in_graph);
         },
-        true, use_st32 ? 8 : 1));
+        true, use_st32 ? loop_copies(o, std::max({A64.box_nx, A64.box_ny, A64.box_nz}), kCopiesM, kCopiesWorthM) : 1));
   } else {
     MultiBufs<double> W{static_cast<double*>(r), static_cast<double*>(p),
                         static_cast<double*>(Ap), nullptr, dst, partials, tickets, err};
