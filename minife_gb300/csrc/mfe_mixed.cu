@@ -51,6 +51,12 @@ constexpr int kCopiesWorth = 16;
 // (mfe_mixed_loop.cu: 124^3 27.7 us per iteration against 29.1 here, 160 x 192 x
 // 144 50 against 40.5)
 constexpr int64_t kLoopRows = 2000000;
+// A round of the loop ends with a read of the state, which only some iterations
+// repay.  Solves with an update every 1 / 2 / 4 iterations, as graph and in rounds:
+// 24^3 3.38, 2.60, 2.22 ms and 4.60, 2.92, 2.13; 64^3 10.7, 7.4, 5.7 and 13.9, 8.2,
+// 5.4; 100^3 22.3, 13.9, 9.6 and 24.8, 14.6, 9.3.  After two rounds in a row of fewer
+// iterations than this the rest runs as a graph.
+constexpr int kShortRound = 4;
 
 // p = r (first) or p = r + beta p, FP32 (cg_solve.hpp:153-161).  The previous
 // iteration's x32 += alpha p (cg_solve.hpp:201-205) is done here, where the
@@ -418,12 +424,17 @@ mfe_status cg_mixed(mfe_ctx* ctx, const mfe_csr* A64_in, const double* b, double
   const bool eager = getenv("MFE_CG_EAGER") != nullptr;
   float w8[8];
   bool loop = !eager && B.stencil && n <= kLoopRows && stencil_mirror_classes(B.coef, w8);
+  int done = 0, short_rounds = 0;
   if (eager || loop) {
     for (;;) {
       MFE_CUDA_TRY(ctx, cudaMemcpyAsync(hs, B.st, sizeof(MixState), cudaMemcpyDeviceToHost, ctx->stream));
       MFE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
       if (!hs->cont || hs->err) break;
       if (loop) {
+        if (hs->updates > 0) short_rounds = hs->k - done < kShortRound ? short_rounds + 1 : 0;
+        done = hs->k;
+        loop = short_rounds < 2;
+        if (!loop) break;
         const mfe_status st = launch_mixed_loop(ctx, &A64, B.coef, B.r, B.p, B.x32, B.Ap, B.st);
         if (st != MFE_OK && st != MFE_NOT_SUPPORTED) return st;
         loop = st == MFE_OK;
