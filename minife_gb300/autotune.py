@@ -9,7 +9,7 @@ workload:
 * tune_mixed (one box): refine_k over 10..50 and the reliable-update drop
   inner_tol;
 * tune_multi (many right-hand sides on one box): the stencil SpMM's z steps
-  per work item, then refine_k and inner_tol.
+  per work item, then refine_k and inner_tol, then the solver's own z steps.
 
 The batch search, in detail:
 
@@ -141,7 +141,8 @@ def tune_multi(A, B, X, tol: float = 1e-8, tol_mode: str = "relative", max_iter:
     """Tune the multi-RHS mixed solve of A X = B (B, X device (n, nrhs)):
     the stencil SpMM's z steps per work item on solves capped at probe_iters
     iterations (the same work for every shape), then refine_k x inner_tol on
-    full solves.  The chosen z_chunk is applied to the context.  Returns
+    full solves, and the best of these once more with the solver's own choice of
+    the z steps (z_chunk 0).  The chosen z_chunk is applied to the context.  Returns
     {"z_chunk", "refine_k", "inner_tol", "solve_seconds", "cached", ...}."""
     import minife_gb300 as M
     key = signature([A.box], "mixed-multi%d" % B.shape[1])
@@ -179,6 +180,16 @@ def tune_multi(A, B, X, tol: float = 1e-8, tol_mode: str = "relative", max_iter:
     best, t, rec2 = _best_full(trials, lambda cfg: solve(cfg, 0), log)
     if best is None:
         best, t = cur, None
+    # the solver's own choice by the box, which also suits the context's later solves
+    M.set_multi_tuning(0)
+    own, ok = solve(best, 0)
+    rec2.append(dict(best, z_chunk=0, seconds=own, stage="full", converged=ok))
+    if log:
+        log("full z_chunk=0: %.4f s" % own)
+    if ok and (t is None or own < t):
+        best, t = dict(best, z_chunk=0), own
+    else:
+        M.set_multi_tuning(best["z_chunk"])
     entry = dict(best, solve_seconds=t, trials=rec + rec2)
     if use_cache:
         _store(key, entry)
