@@ -11,8 +11,8 @@
 // In FP64 that is 13.5 operations per row with p.Ap, and GB300's FP64 pipe
 // takes 1.9 of them per clock and SM: 0.508 ms at 256^3 in the solve, against
 // 0.041 ms for the bytes.  Its integer pipe does 60 multiply-adds of 32 x 32 +
-// 64 bits per clock and SM, so the sums are formed there, to more bits than
-// FP64 keeps:
+// 64 bits per clock and SM, so the sums are formed there, closer to exact in norm
+// than in FP64:
 //
 //   * Every p~ of a plane is split once, as it is staged in shared memory,
 //     into its exponent e and a signed 60-bit integer v (2^7 times the
@@ -30,11 +30,20 @@
 //     to the largest of their planes' E, converts once (round to nearest) and
 //     moves the exponent.
 //
-// The result is within 2^-55 sum |w| max |p~| of exact, the maximum over the
-// thread's windows in three planes, plus one rounding.  Measured against the
-// exact product, relative 2-norm: N(0, 1) vectors 5.6e-17 (the FP64 kernel
-// 1.1e-16), smooth ones 1.2e-15 (7.8e-15: the sums cancel).  The bound is on
-// the window's largest entry and not entry by entry: enough for the CG, whose
+// The result is within 2^-53 sum |w| max |p~| of exact, the maximum over the
+// thread's windows in three planes, plus one rounding: in units of V, 2^-56 of that
+// at most, 1/4 for the entries' floors, 0.85 for the weights' rounding, 4 x 1/4 dropped
+// and 1/2 rounded in each of three plane parts, 2 where exponents are aligned.
+// Measured along CGs of a 64 x 48 x 40 box (iterations 1 to 200; the arithmetic
+// restated on the host against 113 bits), relative 2-norm, and the worst row's part
+// of its own sum |w||p|: N(0, 1) right-hand sides 6e-17 to 8e-17 and 2e-16 to 4e-16
+// (rows in FP64 1.4e-16 to 3.0e-16 and 4e-16 to 5e-16); miniFE's own, whose p falls by
+// orders of magnitude next to the face at 1, 5e-17 to 7e-17 and, in one row in a
+// hundred of the first iterations, up to 5e-14 (8e-17 to 3e-16 and 3e-16).
+// So the product is closer than FP64 in norm, and row by row too where p has no such
+// fronts; a row whose entries all lie 2^k below the window's largest loses k bits
+// (a thread whose positions run over a line's end has both ends in its window).
+// That is enough for the CG, whose
 // scalars mix all of p and which stops on the CSR residual only; a product
 // offered to a caller promises more, so that one (mfe_spmv_stencil64) and the
 // Jacobi PCG's stay on the FP64 kernel.  Rows whose window holds an infinity, a
