@@ -42,6 +42,7 @@ constexpr int kMaxPartM = 2048;
 // reductions (multi_dot_reduce): blocks per group, and what one needs of
 // partials (32 each) and tickets
 constexpr int kGroupM = 32;
+constexpr int kOneGroupM = 256;  // up to so many blocks are one group
 constexpr int kPartsM = kMaxPartM + kMaxPartM / kGroupM;
 constexpr int kTicketsM = 1 + kMaxPartM / kGroupM;
 // iterations in the loop's body with the stencil, and how many a solve must take to
@@ -118,7 +119,10 @@ struct SpmmParams {
 // per warp.  With cg set (out = cg->pAp) the last block also forms cg->alpha.
 // One block summing the partials of all (up to 1,216 x 32 of them) queued
 // 10 us on its SM's FP64 pipe: 64^3 x 32, the r update 33.5 us (cold caches),
-// with the groups 24.1.
+// with the groups 24.1.  Few blocks (kOneGroupM) are one group, as the second level
+// costs 0.6 us per dot: whole solves of 40 iterations, one column, FP64: 10^3 1.04 ms in
+// one group, 1.17 in several; 20^3 (290 blocks) 1.69 with one group up to 256, 1.75
+// up to 128, 1.69 up to 400; 22^3 x 8 2.15, 2.21, 2.24.
 __device__ void multi_dot_reduce(double v, double* red, double* partials, unsigned* ticket,
                                  double* out, int nlanes, MultiState* cg = nullptr)
 {
@@ -145,19 +149,28 @@ __device__ void multi_dot_reduce(double v, double* red, double* partials, unsign
   };
   // `count` sums of 32 from `from` on, into red: the warps take every nw-th
   auto gather = [&](const double* from, int count) {
-    double s = 0.0;
-#pragma unroll 4
-    for (int i = warp; i < count; i += nw) s += __ldcg(&from[(size_t)i * 32 + lane]);
-    red[warp * 32 + lane] = s;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;  // (four loads in flight)
+    int i = warp;
+    for (; i + 3 * nw < count; i += 4 * nw) {
+      s0 += __ldcg(&from[(size_t)i * 32 + lane]);
+      s1 += __ldcg(&from[(size_t)(i + nw) * 32 + lane]);
+      s2 += __ldcg(&from[(size_t)(i + 2 * nw) * 32 + lane]);
+      s3 += __ldcg(&from[(size_t)(i + 3 * nw) * 32 + lane]);
+    }
+    for (; i < count; i += nw) s0 += __ldcg(&from[(size_t)i * 32 + lane]);
+    red[warp * 32 + lane] = (s0 + s1) + (s2 + s3);
   };
-  const int g = (int)blockIdx.x / kGroupM, ng = ((int)gridDim.x + kGroupM - 1) / kGroupM;
-  const int members = min(kGroupM, (int)gridDim.x - g * kGroupM);
+  const int size = (int)gridDim.x <= kOneGroupM ? (int)gridDim.x : kGroupM;
+  const int g = (int)blockIdx.x / size, ng = ((int)gridDim.x + size - 1) / size;
+  const int members = min(size, (int)gridDim.x - g * size);
   double* const groups = partials + (size_t)kMaxPartM * 32;
   red[warp * 32 + lane] = v;
   if (!publish(partials + (size_t)blockIdx.x * 32, ticket + 1 + g, (unsigned)members)) return;
-  gather(partials + (size_t)g * kGroupM * 32, members);
-  if (!publish(groups + (size_t)g * 32, ticket, (unsigned)ng)) return;
-  gather(groups, ng);
+  gather(partials + (size_t)g * size * 32, members);
+  if (ng > 1) {
+    if (!publish(groups + (size_t)g * 32, ticket, (unsigned)ng)) return;
+    gather(groups, ng);
+  }
   __syncthreads();
   if (threadIdx.x < nlanes) {
     double s = 0.0;
