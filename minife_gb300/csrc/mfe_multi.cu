@@ -42,7 +42,7 @@ constexpr int kMaxPartM = 2048;
 // reductions (multi_dot_reduce): blocks per group, and what one needs of
 // partials (32 each) and tickets
 constexpr int kGroupM = 32;
-constexpr int kOneGroupM = 256;  // up to so many blocks are one group
+constexpr int kOneGroupM = 160;  // up to so many blocks are one group
 constexpr int kPartsM = kMaxPartM + kMaxPartM / kGroupM;
 constexpr int kTicketsM = 1 + kMaxPartM / kGroupM;
 // iterations in the loop's body with the stencil, and how many a solve must take to
@@ -120,9 +120,9 @@ struct SpmmParams {
 // One block summing the partials of all (up to 1,216 x 32 of them) queued
 // 10 us on its SM's FP64 pipe: 64^3 x 32, the r update 33.5 us (cold caches),
 // with the groups 24.1.  Few blocks (kOneGroupM) are one group, as the second level
-// costs 0.6 us per dot: whole solves of 40 iterations, one column, FP64: 10^3 1.04 ms in
-// one group, 1.17 in several; 20^3 (290 blocks) 1.69 with one group up to 256, 1.75
-// up to 128, 1.69 up to 400; 22^3 x 8 2.15, 2.21, 2.24.
+// costs 0.6 us per dot: whole solves of 40 iterations in FP64, always in groups of 32 /
+// one group up to 160 / 256: 14^3 x 1 1.46, 1.37, 1.37 ms; 22^3 x 4 2.12, 2.09, 2.13; 24^3
+// x 4 2.43, 2.40, 2.47.
 __device__ void multi_dot_reduce(double v, double* red, double* partials, unsigned* ticket,
                                  double* out, int nlanes, MultiState* cg = nullptr)
 {
@@ -149,16 +149,21 @@ __device__ void multi_dot_reduce(double v, double* red, double* partials, unsign
   };
   // `count` sums of 32 from `from` on, into red: the warps take every nw-th
   auto gather = [&](const double* from, int count) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;  // (four loads in flight)
+    double s = 0.0;
     int i = warp;
-    for (; i + 3 * nw < count; i += 4 * nw) {
-      s0 += __ldcg(&from[(size_t)i * 32 + lane]);
-      s1 += __ldcg(&from[(size_t)(i + nw) * 32 + lane]);
-      s2 += __ldcg(&from[(size_t)(i + 2 * nw) * 32 + lane]);
-      s3 += __ldcg(&from[(size_t)(i + 3 * nw) * 32 + lane]);
+    if (count > 2 * kGroupM) {  // (four sums side by side, where there are many)
+      double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      for (; i + 3 * nw < count; i += 4 * nw) {
+        s += __ldcg(&from[(size_t)i * 32 + lane]);
+        s1 += __ldcg(&from[(size_t)(i + nw) * 32 + lane]);
+        s2 += __ldcg(&from[(size_t)(i + 2 * nw) * 32 + lane]);
+        s3 += __ldcg(&from[(size_t)(i + 3 * nw) * 32 + lane]);
+      }
+      s = (s + s1) + (s2 + s3);
     }
-    for (; i < count; i += nw) s0 += __ldcg(&from[(size_t)i * 32 + lane]);
-    red[warp * 32 + lane] = (s0 + s1) + (s2 + s3);
+#pragma unroll 4
+    for (; i < count; i += nw) s += __ldcg(&from[(size_t)i * 32 + lane]);
+    red[warp * 32 + lane] = s;
   };
   const int size = (int)gridDim.x <= kOneGroupM ? (int)gridDim.x : kGroupM;
   const int g = (int)blockIdx.x / size, ng = ((int)gridDim.x + size - 1) / size;
