@@ -160,7 +160,7 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // Measured there, us per call: a pass for the longest row, two stages and 27
 // FMAs 121; without the pass 107; in pairs 103; one stage, 16 / 20 / 24 warps per
 // SM 86 / 79 / 76 (50 are the bytes at the HBM rate).  Rows of 27 entries (no
-// pairs): 135 / 111; of 5: 126 / 69; of 20 to 40: 700 / 144.  Cutting a
+// pairs): 135 / 110; of 5: 126 / 69; of 20 to 40: 700 / 141.  Cutting a
 // group's entries into 32 equal runs, a lane per run, took twice the
 // instructions, 147 us.  FP32 rows (no pairs) against 128-row tiles behind block
 // barriers, 1.48 M rows of 27 / of 4 to 27: longest row stated 68, 65 before and
@@ -168,10 +168,10 @@ __host__ __device__ constexpr int stg_cap(int max_len, bool ell)
 // Rows whose lengths come in regions (half of them 4 to 7, half 27 to 32, so that
 // every group of the second half is larger than the stage), FP64 / FP32: with the
 // longest row known and a stage for it 133 / 73; such groups a row at a time over
-// the warp 342 / 371; in parts 98 / 71.  Rows of 8 and 56 in turn 737 / 262 (a warp
-// per row), 714 / 663 (a row at a time), 254 / 128; one row of 200 among 31 of 10 930
-// / 465, 585 / 653, 317 / 111.  One row of 200,000 among rows of 20 takes 2990 / 1706
-// (a warp per row), 990 / 550.
+// the warp 342 / 371; in parts 97 / 72.  Rows of 8 and 56 in turn 737 / 262 (a warp
+// per row), 714 / 663 (a row at a time), 235 / 125; one row of 200 among 31 of 10 930
+// / 465, 585 / 653, 241 / 97.  One row of 200,000 among rows of 20 takes 2990 / 1706
+// (a warp per row), 1030 / 560.
 constexpr int kAnyLongest = 54;
 constexpr int kAnyWarps = 24;  // per SM, in blocks of W
 
@@ -255,7 +255,9 @@ template <typename T>
 __device__ __forceinline__ T strided_dot(const T* gv, const int32_t* gc, int k, int end, int L, int any,
                                          const T* __restrict__ x)
 {
-  constexpr int kBatch = 9;  // gathers in flight
+  // gathers in flight (nine: rows of 8 and 56 in turn 254 us, and the registers cost the
+  // other groups 0.7 %)
+  constexpr int kBatch = 4;
   T s = T(0);
   for (; __any_sync(0xffffffffu, k < end); k += kBatch * L) {
     T v[kBatch], xv[kBatch];
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(W * 32, kAnyWarps / W) k_spmv_any(SpmvParams<T
     T sum = T(0);
     const bool whole = staged(a, e);
     const int longest = __reduce_max_sync(0xffffffffu, en - st);
-    if (whole && longest <= kAnyLongest) {
+    if (__builtin_expect(whole && longest <= kAnyLongest, 1)) {
       const T* gv = dv + (a & (VA - 1));
       const int32_t* gc = dc + (a & 3);
       if constexpr (sizeof(T) == 8) {
