@@ -11,10 +11,13 @@ Keys beyond the base contract:
   e2e          the same solve through the host drop-in call
                (mfe_cg_solve_host: host CSR and b in pinned memory copied to the
                device inside the timed region, x copied back)
-  roofline     the dominant kernel (the verified FP64 stencil SpMV) timed with
-               CUDA events on its stream against the measured FP64 pipe rate,
-               its HBM fraction beside it; traffic from the committed ncu
-               summary.  fp64_csr_values carries the same solve with the CSR
+  roofline     one iteration of the headline solve (the stencil product in fixed
+               point, the update and the p update) against HBM: its 88 bytes per
+               row over the solve's time per iteration.  stencil64 in it: the
+               same operator as a product of its own (mfe_spmv_stencil64, FP64)
+               timed with CUDA events against the measured FP64 pipe rate, its
+               HBM fraction beside it, traffic from the committed ncu summary.
+               fp64_csr_values carries the same solve with the CSR
                values and the box CSR SpMV's roofline against HBM.
   cpu_baseline the OpenMP CG port (oracle/cpu_baseline.c) on the host cores:
                one whole solve of the same system to the same tolerance
@@ -303,9 +306,9 @@ def run_gpu(args):
     d_ops = float((x - x_csr).norm() / x_csr.norm())
     del x_csr
 
-    # dominant kernels timed alone on the same stream with CUDA events: the
-    # FP64 stencil SpMV of the headline solve and the CSR SpMV (with its
-    # fused p.Ap in the CSR solve)
+    # kernels timed alone on the same stream with CUDA events: the FP64 stencil
+    # SpMV (the headline solve applies the operator in fixed point instead) and
+    # the CSR SpMV (with its fused p.Ap in the CSR solve)
     p = torch.randn(n, dtype=torch.float64, device="cuda")
     Ap = torch.empty_like(p)
     S = M.Stencil64(A)
@@ -511,17 +514,27 @@ def run_gpu(args):
             "multi_rhs": multi,
             "adjoint": adjoint,
             "small_30cubed": small,
-            "roofline": {"bound": "fp64", "achieved": st_ops / t_st / 1e9,
-                         "peak": FP64_PEAK_TFLOPS / 2 * 1e3, "unit": "G FP64 op/s",
-                         "frac": st_ops / t_st / 1e9 / (FP64_PEAK_TFLOPS / 2 * 1e3),
-                         "traffic": traffic_from_profile("st64_bytes_per_launch_256"),
-                         "kernel": "k_spmv_st64 (verified FP64 stencil SpMV, 12.5 FP64 operations "
-                                   "per row without the fused dot)",
-                         "kernel_ms": t_st * 1e3, "algorithmic_ops": st_ops,
-                         "peak_kind": "measured (FP64 FMA-only kernel, one operation per FMA)",
-                         "hbm": {"achieved_gbs": st_bytes / t_st / 1e9, "peak_gbs": peak,
-                                 "frac": st_bytes / t_st / 1e9 / peak,
-                                 "algorithmic_bytes": st_bytes}},
+            "roofline": {"bound": "hbm", "achieved": iter_bytes_st * res.num_iters / t_step / 1e9,
+                         "peak": peak, "unit": "GB/s",
+                         "frac": iter_bytes_st * res.num_iters / t_step / 1e9 / peak,
+                         "traffic": None,
+                         "kernel": "one CG iteration: k_spmv_fixed (the verified stencil in fixed "
+                                   "point with p.Ap), k_cg_update, k_cg_p",
+                         "kernel_ms": t_step / res.num_iters * 1e3,
+                         "algorithmic_bytes": iter_bytes_st,
+                         "peak_kind": peak_kind + " (HBM copy)",
+                         "stencil64": {
+                             "bound": "fp64", "achieved": st_ops / t_st / 1e9,
+                             "peak": FP64_PEAK_TFLOPS / 2 * 1e3, "unit": "G FP64 op/s",
+                             "frac": st_ops / t_st / 1e9 / (FP64_PEAK_TFLOPS / 2 * 1e3),
+                             "traffic": traffic_from_profile("st64_bytes_per_launch_256"),
+                             "kernel": "k_spmv_st64 (verified FP64 stencil SpMV, 12.5 FP64 "
+                                       "operations per row without the fused dot)",
+                             "kernel_ms": t_st * 1e3, "algorithmic_ops": st_ops,
+                             "peak_kind": "measured (FP64 FMA-only kernel, one operation per FMA)",
+                             "hbm": {"achieved_gbs": st_bytes / t_st / 1e9, "peak_gbs": peak,
+                                     "frac": st_bytes / t_st / 1e9 / peak,
+                                     "algorithmic_bytes": st_bytes}}},
             "e2e": e2e,
             "cpu_baseline": cpu,
             "gpu_launches": gpu_launches,

@@ -239,9 +239,9 @@ mfe_status mfe_dot_f32(mfe_ctx* ctx, int64_t n, const float* x, const float* y,
                        double* result);
 
 /* Fault injection for tests of the bounded-wait error path; no counterpart
- * in the reference.  The next SpMV with a shared-memory staging ring (the
- * box-structured kernel, or the warp-staged kernels of an FP64 CSR with rows
- * of at most 32 entries and of the ELL matrix) launched on ctx outside a
+ * in the reference.  The next SpMV with shared-memory stages (the
+ * box-structured kernel, or the warp-staged kernels of a CSR, FP64 or FP32, with
+ * rows of at most 32 entries and of the ELL matrix) launched on ctx outside a
  * graph capture issues none of its copies, so its bounded waits run out
  * after wait_ns nanoseconds (1 ms .. 2 s) with no copy in flight; the call
  * that launched it returns MFE_TIMEOUT (a solve) or mfe_synchronize does

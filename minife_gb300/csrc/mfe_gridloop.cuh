@@ -157,8 +157,8 @@ inline mfe_status start_sync(mfe_ctx* ctx, unsigned* arrived, GridSync* sync)
 // 181, 156); 16^3 519, 292, 225, 189 (515, 373, 374, 371; 1040, 563, 295, 263); mixed
 // 24^3 939, 505, 392, 366 (982, 736, 690, 677; 1451, 1369, 1080, 910).  Loops that fill
 // the device go one after another: 30^3 916, 848, 784, 772, where graphs take 2303,
-// 1154, 621, 555 (with more than two threads the graphs' gaps fill up); 64^3 3641,
-// 3579, 3513, 3533 (7519, 5110, 4011, 3990).
+// 1154, 621, 555 (with more than two threads the graphs' gaps fill up; 24^3 to 52^3
+// are so); 64^3 3641, 3579, 3513, 3533 (7519, 5110, 4011, 3990).
 struct LoopOrder {
   struct Loop {
     cudaEvent_t end;

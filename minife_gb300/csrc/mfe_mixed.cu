@@ -20,13 +20,14 @@
 //
 // One iteration is three kernels (k_mx_p, the FP32 operator with p.Ap -- the
 // verified stencil of mfe_stencil.cu or the box SpMV over an FP32 copy of
-// the values -- and k_mx_update) plus two that only work when an update is
-// due (the graph cannot branch cheaply per iteration, so k_mx_xupdate and the
-// FP64 residual SpMV check a device-side gate and return at once when it is
-// closed) and a one-thread bookkeeping kernel that sets the loop condition.
-// The whole solve is one CUDA graph launch with a conditional while node; small
-// boxes on the stencil run the iterations up to a reliable update in one
-// cooperative kernel instead (mfe_mixed_loop.cu).
+// the values -- and k_mx_update, which decides whether an update is due and
+// else sets the loop condition).  The update (k_mx_xupdate, the FP64 residual SpMV
+// and a one-thread bookkeeping kernel) sits in a conditional node that is entered
+// when it is due.  The whole solve is one CUDA graph launch with a conditional while
+// node, whose body holds several iterations where the solve is expected to repay
+// them (loop_copies); small boxes on the stencil run the iterations up to a reliable
+// update in one cooperative kernel instead (mfe_mixed_loop.cu), unless the updates
+// come every few iterations.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
