@@ -21,6 +21,7 @@ LOOPS = [((9, 8, 7), dict(f64_operator="csr")), ((30, 30, 30), dict(f64_operator
 @pytest.mark.parametrize("dims,kw", LOOPS)
 def test_timeout(dims, kw):
     ctx = M.Context()
+    ctx.bind_torch_stream()
     A, b = M.build_system(*dims, ctx=ctx)
     kw = dict(kw, max_iter=3000, tol=1e-9, tol_mode="relative", ctx=ctx)
     x = torch.zeros_like(b)
@@ -44,6 +45,7 @@ def test_refused(dims, kw):
     # end within the tolerance: ||A (x - y)|| <= 2 tol ||b|| up to the products'
     # rounding (28 2^-53 of the row sums |A||x| each)
     ctx = M.Context()
+    ctx.bind_torch_stream()
     A, b0 = M.build_system(*dims, ctx=ctx)
     g = torch.Generator(device="cuda")
     g.manual_seed(2)

@@ -54,6 +54,7 @@ def test_regions(shape, n, dtype, unit):
     np.add.at(exact, rows, prod)
     np.add.at(size, rows, np.abs(prod))
     ctx = M.Context()
+    ctx.bind_torch_stream()
     # the longest row unknown, or stated where that keeps the kernel
     for stated in [0] + ([int(lens.max())] if lens.max() <= 32 else []):
         A = M.CSRMatrix(*dev[:3], max_row_len=stated)

@@ -38,6 +38,7 @@ def test_right_length(n, length, stated):
     (ro, cols, vals, x), exact, bound = system(np.full(n, length), 1)
     A = M.CSRMatrix(ro, cols, vals, max_row_len=stated)
     ctx = M.Context()
+    ctx.bind_torch_stream()
     y = torch.full_like(x, 7.0)
     M.matvec(A, x, y, ctx=ctx)
     ctx.synchronize()
@@ -62,6 +63,7 @@ def test_stated_too_short(rest, stated, refused):
     (ro, cols, vals, x), exact, bound = system(np.where(i % 128 < 32, 27, rest), 2)
     A = M.CSRMatrix(ro, cols, vals, max_row_len=stated)
     ctx = M.Context()
+    ctx.bind_torch_stream()
     y = torch.full_like(x, 7.0)
     M.matvec(A, x, y, ctx=ctx)
     if refused:
@@ -82,6 +84,7 @@ def test_box_with_unaligned_x():
     off = torch.randn(A.nrows + 1, device="cuda", dtype=F32, generator=g)[1:]
     assert off.data_ptr() % 16
     ctx = M.Context()
+    ctx.bind_torch_stream()
     y, ref = torch.empty(A.nrows, device="cuda", dtype=F32), torch.empty_like(b)
     M.matvec(A32, off, y, ctx=ctx)
     ctx.synchronize()
