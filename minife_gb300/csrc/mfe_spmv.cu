@@ -683,11 +683,16 @@ static int any_cap(int64_t n, int64_t nnz, int max_len)
 // read the same part of x: FP32 rows of columns within 3,000 of the diagonal, whose
 // large stages leave little L1, 600,000 rows of 27 to 32 / 20 to 32 / 27 entries,
 // blocks of two 119, 113, 110 us, of eight 93, 85, 87 (with columns within 30 even).
-// FP64 rows and short ones keep two (1.48 M FP64 rows of 4 to 27: 75.6 and 77.6).
+// FP64 rows and short ones keep two (1.48 M FP64 rows of 4 to 27: 75.6 and 77.6), and so
+// do matrices of fewer than four groups a warp, whose last ones are then unevenly
+// spread over the SMs (rows of 27, columns near the diagonal: 30^3 2.96 and 3.01 us,
+// 52^3 5.50 and 6.14, 70^3 9.20 and 9.40, 100^3 38.2 and 38.2; the last groups of all warps
+// dealt out over the blocks 52^3 5.76, 70^3 9.71, and FP64 rows slower by 1 %).
 template <typename T>
-static int any_warps(int cap)
+static int any_warps(const mfe_ctx* ctx, int64_t nrows, int cap)
 {
-  return sizeof(T) == 4 && cap > 25 * 32 ? 8 : 2;  // a mean row of 19 entries or more
+  // (a stage of more than 25 entries a row: a mean row of 19 or more)
+  return sizeof(T) == 4 && cap > 25 * 32 && nrows >= (int64_t)4 * 32 * kAnyWarps * ctx->sm_count ? 8 : 2;
 }
 
 template <typename T>
@@ -699,7 +704,7 @@ static size_t any_smem(int cap, int warps)
 template <typename T>
 static int any_grid(mfe_ctx* ctx, int64_t nrows, int cap)
 {
-  const int W = any_warps<T>(cap);
+  const int W = any_warps<T>(ctx, nrows, cap);
   const int per_sm = std::max(1, std::min(kAnyWarps / W, (int)((228 * 1024) / (any_smem<T>(cap, W) + 1024 + 256 * W))));
   return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(nrows, (int64_t)32), (int64_t)W),
                                                      (int64_t)ctx->sm_count * per_sm));
@@ -722,7 +727,7 @@ static mfe_status launch_any(mfe_ctx* ctx, SpmvParams<T>& P, int max_len)
   const int most = max_len > 0 ? stated_most(kCheckRows<T>, max_len) : INT_MAX;
   MFE_TRY(take_wait_injection(ctx, &P.withhold_ns));
   if constexpr (sizeof(T) == 4) {
-    if (any_warps<T>(cap) == 8) return launch_any_w<T, MODE, 8>(ctx, P, cap, most);
+    if (any_warps<T>(ctx, P.n, cap) == 8) return launch_any_w<T, MODE, 8>(ctx, P, cap, most);
   }
   return launch_any_w<T, MODE, 2>(ctx, P, cap, most);
 }

@@ -1,6 +1,6 @@
 """FP32 CSR products on both sides of the mean row length (19) from which a block has
 eight warps instead of two, at row numbers around a block's share (64 and 256 rows)
-and past one wave of blocks.
+and around those (four groups a warp of 152 SMs) from which they may be eight.
 
 Bound as in test_gpu_spmv_any: (len + 32) 2^-24 sum |a||x|."""
 import numpy as np
@@ -16,7 +16,7 @@ import minife_gb300 as M  # noqa: E402
 
 
 @pytest.mark.parametrize("length", [17, 18, 19, 20, 27, 32])
-@pytest.mark.parametrize("n", [1, 63, 65, 255, 257, 152 * 3 * 256 + 33])
+@pytest.mark.parametrize("n", [1, 63, 65, 255, 257, 4 * 32 * 24 * 152 - 1, 4 * 32 * 24 * 152, 4 * 32 * 24 * 152 + 257])
 def test_rows(n, length):
     rng = np.random.default_rng(length)
     lens = np.clip(rng.integers(length - 2, length + 3, n), 1, 32)
